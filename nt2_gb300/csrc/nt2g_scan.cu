@@ -13,23 +13,21 @@
 // NT2 policy: one thread per segment in that order with NT2's unfused float
 // operations: bit-identical wherever NT2 spreads segments over threads.
 //
-// Fast policy, three phases with no block waiting on another:
-//   1. each chunk of each segment reduces to an aggregate,
-//   2. per segment, the chunk aggregates are scanned in order (exclusive),
-//   3. each chunk is scanned again, starting from its prefix.
-// Contiguous segments (lo = 1) run one warp per chunk in tiles of 512
-// elements (16 consecutive ones per lane, an in-order warp scan of the lane
-// totals);
-// phase 1 of cumsum/cumprod is a plain reduction (order does not matter to a
-// commutative aggregate).  Strided segments run one thread per segment (four
-// with float4) over chunks of the scan range, 8 rows of loads at a time.  cumsum carries compensated sums (s + c; chunk prefixes in
-// FP64), so each output is within about an ulp of the exact prefix; cumprod
-// carries FP64 products; cummax/cummin are exact: NT2's (s > x) ? s : x is
-// not associative once a NaN appears (a NaN summary is replaced by the next
-// element), so each element is a pair (value, starts-a-segment) with NaN
-// elements starting segments, which makes the in-order combine associative
-// and reproduces NT2's sequential result, NaNs included.  When a segment fits
-// one chunk, phase 3 alone runs.
+// Fast policy, with no block waiting on another:
+//  * enough segments to fill the GPU with one worker each: one pass, a worker
+//    walking its segment with a carry (contiguous segments: a block, short
+//    ones sharing it; strided ones: a thread);
+//  * else segments are cut into chunks: a first kernel folds each chunk to an
+//    aggregate, a second one scans each chunk from the in-order sum of the
+//    aggregates before it.  The first walks its chunks backwards, so that the
+//    second, walking forwards, finds what was read last in L2.
+// cumsum carries compensated sums (s + c; chunk prefixes in FP64), so each
+// output is within about an ulp of the exact prefix; cumprod carries FP64
+// products; cummax/cummin are exact: NT2's (s > x) ? s : x is not associative
+// once a NaN appears (a NaN summary is replaced by the next element), so each
+// element is a pair (value, starts-a-segment) with NaN elements starting
+// segments, which makes the in-order combine associative and reproduces NT2's
+// sequential result, NaNs included.
 #include "nt2g_accum.cuh"
 #include "nt2g_common.cuh"
 #include "nt2g_internal.h"
@@ -37,7 +35,11 @@
 namespace nt2g {
 
 constexpr int kScanThreads = 256;
-constexpr int64_t kScanChunk = 16384;  // multiple of the 512-element tile
+constexpr int kLineThreads = 128, kRun = 33;       // contiguous tiles: 128 threads of up to 33 elements
+constexpr int kTileMax = kLineThreads * kRun;      // 17 KB of shared memory, 13 blocks an SM
+constexpr int64_t kPackBelow = 1024;               // segments shorter than this share tiles
+constexpr int64_t kLineChunks = 152 * 12;          // chunks (blocks) a contiguous scan is cut into at least
+constexpr int64_t kInlinePrefix = 64;              // strided chunks whose prefix the scan itself adds up
 constexpr int64_t kScanTarget = 152 * 1024;
 
 // ------------------------------------------------------------- elements --
@@ -48,7 +50,6 @@ template <int OP> struct SE {
     float v;
     int h;
     __device__ static SE id() { return SE{OP == NT2G_SCAN_MAX ? -INFINITY : INFINITY, 2}; }
-    __device__ static SE of(float x) { return SE{x, x != x ? 1 : 0}; }
     __device__ static float op(float s, float x)
     {
         return OP == NT2G_SCAN_MAX ? ((s > x) ? s : x) : ((s < x) ? s : x);
@@ -59,18 +60,23 @@ template <int OP> struct SE {
         if (a.h & 2) return SE{op(a.v, b.v), b.h};  // the neutral value meets the first element
         return (b.h & 1) ? b : SE{op(a.v, b.v), a.h};
     }
+    // combine(*this, of(x)): whatever the flags, the value is NT2's step
+    __device__ void push(float x)
+    {
+        v = op(v, x);
+        h = (x != x) | (h & 1);
+    }
     __device__ float out() const { return v; }
     __device__ SE shfl_up(int off) const
     {
         return SE{__shfl_up_sync(0xffffffffu, v, off), __shfl_up_sync(0xffffffffu, h, off)};
     }
-    __device__ SE shfl(int lane) const { return SE{__shfl_sync(0xffffffffu, v, lane), __shfl_sync(0xffffffffu, h, lane)}; }
 };
 // SUM: compensated pair
 template <> struct SE<NT2G_SCAN_SUM> {
     CSum v;
     __device__ static SE id() { return SE{CSum{0.0f, 0.0f}}; }
-    __device__ static SE of(float x) { return SE{CSum{x, 0.0f}}; }
+    __device__ void push(float x) { csum_add(v, x); }
     __device__ static SE combine(const SE &a, const SE &b)  // a precedes b
     {
         SE r = a;
@@ -88,25 +94,20 @@ template <> struct SE<NT2G_SCAN_SUM> {
     {
         return SE{CSum{__shfl_up_sync(0xffffffffu, v.s, off), __shfl_up_sync(0xffffffffu, v.c, off)}};
     }
-    __device__ SE shfl(int lane) const
-    {
-        return SE{CSum{__shfl_sync(0xffffffffu, v.s, lane), __shfl_sync(0xffffffffu, v.c, lane)}};
-    }
 };
 // PROD: double
 template <> struct SE<NT2G_SCAN_PROD> {
     double v;
     __device__ static SE id() { return SE{1.0}; }
-    __device__ static SE of(float x) { return SE{(double)x}; }
+    __device__ void push(float x) { v *= (double)x; }
     __device__ static SE combine(const SE &a, const SE &b) { return SE{a.v * b.v}; }
     __device__ float out() const { return (float)v; }
     __device__ double agg() const { return v; }
     __device__ static SE from(double p) { return SE{p}; }
     __device__ SE shfl_up(int off) const { return SE{__shfl_up_sync(0xffffffffu, v, off)}; }
-    __device__ SE shfl(int lane) const { return SE{__shfl_sync(0xffffffffu, v, lane)}; }
 };
 
-// 16-byte chunk record in the workspace: an aggregate, later its prefix
+// 16-byte chunk record in the workspace: an aggregate, later (k_scan_prefix*) its prefix
 struct ScanRec {
     double d;  // SUM, PROD
     float v;   // MAX, MIN
@@ -125,185 +126,7 @@ template <int OP> __device__ __forceinline__ SE<OP> from_rec(const ScanRec &r)
     else return SE<OP>{r.v, r.h};
 }
 
-// In-order inclusive warp scan of one value per lane.
-template <int OP> __device__ __forceinline__ SE<OP> warp_scan(SE<OP> x, int lane)
-{
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-        SE<OP> o = x.shfl_up(off);
-        if (lane >= off) x = SE<OP>::combine(o, x);
-    }
-    return x;
-}
-
-// ----------------------------------------- contiguous segments (lo == 1) --
-// One warp per (segment, chunk): tiles of 512 elements, lane l owning
-// elements 16l..16l+15 of the tile.  PHASE 1 keeps the running carry and stores
-// the chunk aggregate; PHASE 3 starts from the chunk's prefix (or the
-// identity when there is one chunk) and writes every inclusive value.
-template <int OP, int PHASE>
-__global__ void __launch_bounds__(kScanThreads) k_scan_inner(const float *x, int64_t inner, int64_t hi,
-                                                             int64_t chunk, int64_t q, int vec,
-                                                             ScanRec *__restrict__ rec, float *out)
-{
-    const int lane = threadIdx.x & 31;
-    const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t item = warp; item < hi * q; item += nwarps) {
-        const int64_t seg = item / q, c = item - seg * q;
-        const int64_t k0 = c * chunk, k1 = (k0 + chunk < inner) ? k0 + chunk : inner;
-        const float *p = x + seg * inner;
-        float *o = out + seg * inner;
-        if constexpr (PHASE == 1 && (OP == NT2G_SCAN_SUM || OP == NT2G_SCAN_PROD)) {
-            // the chunk aggregate of a commutative operation needs no scan: each
-            // lane folds its float4s (8 in flight), then the lanes combine in order
-            CSum acc{0.0f, 0.0f};
-            double prod = 1.0;
-            for (int64_t t0 = k0; t0 < k1; t0 += 1024) {
-                float f[8][4];
-                int nn[8];
-#pragma unroll
-                for (int u = 0; u < 8; ++u) {
-                    const int64_t e = t0 + 128 * u + 4 * lane;
-                    nn[u] = (int)(k1 - e < 4 ? (k1 - e > 0 ? k1 - e : 0) : 4);
-                    if (vec && nn[u] == 4) {
-                        const float4 v = ld_stream((const float4 *)(p + e));
-                        f[u][0] = v.x; f[u][1] = v.y; f[u][2] = v.z; f[u][3] = v.w;
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) f[u][j] = j < nn[u] ? p[e + j] : 0.0f;
-                    }
-                }
-#pragma unroll
-                for (int u = 0; u < 8; ++u)
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        if (OP == NT2G_SCAN_SUM) csum_add(acc, f[u][j]);
-                        else if (j < nn[u]) prod *= (double)f[u][j];
-                    }
-            }
-            if (OP == NT2G_SCAN_SUM) {
-                acc = warp_csum(acc);
-                if (lane == 0) rec[item] = ScanRec{(double)acc.s + (double)acc.c, 0.0f, 0};
-            } else {
-#pragma unroll
-                for (int off = 16; off; off >>= 1) prod *= __shfl_down_sync(0xffffffffu, prod, off);
-                if (lane == 0) rec[item] = ScanRec{prod, 0.0f, 0};
-            }
-            continue;
-        }
-        SE<OP> carry = (PHASE == 3 && q > 1) ? from_rec<OP>(rec[item]) : SE<OP>::id();
-        // tiles of 512 elements, 16 consecutive ones per lane: the lane folds its
-        // run, one in-order warp scan of the lane totals gives every lane its
-        // prefix, and the lane's outputs follow in order from that prefix
-        for (int64_t t0 = k0; t0 < k1; t0 += 512) {
-            const int64_t e0 = t0 + 16 * lane;
-            const int cnt = (int)(k1 - e0 < 16 ? (k1 - e0 > 0 ? k1 - e0 : 0) : 16);
-            float f[16];
-            if (vec && cnt == 16) {
-#pragma unroll
-                for (int v = 0; v < 4; ++v) {
-                    const float4 w = ld_stream((const float4 *)(p + e0) + v);
-                    f[4 * v] = w.x; f[4 * v + 1] = w.y; f[4 * v + 2] = w.z; f[4 * v + 3] = w.w;
-                }
-            } else {
-#pragma unroll
-                for (int j = 0; j < 16; ++j) f[j] = j < cnt ? p[e0 + j] : 0.0f;
-            }
-            SE<OP> agg = SE<OP>::id();
-#pragma unroll
-            for (int j = 0; j < 16; ++j)
-                if (j < cnt) agg = SE<OP>::combine(agg, SE<OP>::of(f[j]));
-            const SE<OP> inc = warp_scan<OP>(agg, lane);
-            SE<OP> ex = inc.shfl_up(1);
-            if (lane == 0) ex = SE<OP>::id();
-            if (PHASE == 3) {
-                SE<OP> run = SE<OP>::combine(carry, ex);
-                float r[16];
-#pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    run = SE<OP>::combine(run, SE<OP>::of(f[j]));
-                    r[j] = run.out();
-                }
-                if (vec && cnt == 16) {
-#pragma unroll
-                    for (int v = 0; v < 4; ++v)
-                        st_stream((float4 *)(o + e0) + v, make_float4(r[4 * v], r[4 * v + 1], r[4 * v + 2], r[4 * v + 3]));
-                } else {
-#pragma unroll
-                    for (int j = 0; j < 16; ++j)
-                        if (j < cnt) o[e0 + j] = r[j];
-                }
-            }
-            carry = SE<OP>::combine(carry, inc.shfl(31));
-        }
-        if (PHASE == 1 && lane == 0) rec[item] = to_rec<OP>(carry);
-    }
-}
-
-// ---------------------------------------------- strided scans (lo > 1) --
-// Thread per segment (VEC: four neighbouring segments via float4) over the
-// chunk [c*ck, min((c+1)*ck, inner)) of the scan range; grid.y = chunk.
-template <int OP, int VEC, int PHASE>
-__global__ void __launch_bounds__(kScanThreads) k_scan_outer(const float *x, int64_t lo, int64_t inner,
-                                                             int64_t hi, int64_t ck, int64_t q,
-                                                             ScanRec *__restrict__ rec, float *out)
-{
-    const int64_t lv = lo / VEC;
-    const int64_t c = blockIdx.y;
-    const int64_t k0 = c * ck, k1 = (k0 + ck < inner) ? k0 + ck : inner;
-    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < lv * hi; t += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t h = t / lv, l = (t - h * lv) * VEC;
-        const int64_t base = l + lo * inner * h;
-        SE<OP> carry[VEC];
-#pragma unroll
-        for (int v = 0; v < VEC; ++v) {
-            const int64_t seg = l + v + lo * h;
-            carry[v] = (PHASE == 3 && q > 1) ? from_rec<OP>(rec[c * lo * hi + seg]) : SE<OP>::id();
-        }
-        // groups of kGroup rows: all loads of a group are issued before its scan
-        constexpr int kGroup = (OP == NT2G_SCAN_PROD && VEC == 4) ? 4 : 8;  // FP64 products: fewer registers free
-        auto step = [&](int64_t k, const float (&e)[VEC]) {
-            float r[VEC];
-#pragma unroll
-            for (int v = 0; v < VEC; ++v) {
-                carry[v] = SE<OP>::combine(carry[v], SE<OP>::of(e[v]));
-                r[v] = carry[v].out();
-            }
-            if (PHASE == 3) {
-                if constexpr (VEC == 4) st_stream((float4 *)(out + base + lo * k), make_float4(r[0], r[1], r[2], r[3]));
-                else out[base + lo * k] = r[0];
-            }
-        };
-        auto fetch = [&](int64_t k, float (&e)[VEC]) {
-            if constexpr (VEC == 4) {
-                const float4 f = ld_stream((const float4 *)(x + base + lo * k));
-                e[0] = f.x; e[1] = f.y; e[2] = f.z; e[3] = f.w;
-            } else {
-                e[0] = ld_stream(x + base + lo * k);
-            }
-        };
-        int64_t k = k0;
-        for (; k + kGroup <= k1; k += kGroup) {
-            float e[kGroup][VEC];
-#pragma unroll
-            for (int g = 0; g < kGroup; ++g) fetch(k + g, e[g]);
-#pragma unroll
-            for (int g = 0; g < kGroup; ++g) step(k + g, e[g]);
-        }
-        for (; k < k1; ++k) {
-            float e[VEC];
-            fetch(k, e);
-            step(k, e);
-        }
-        if (PHASE == 1) {
-#pragma unroll
-            for (int v = 0; v < VEC; ++v) rec[c * lo * hi + (l + v + lo * h)] = to_rec<OP>(carry[v]);
-        }
-    }
-}
-
-// Chunk records combine in FP64 (sum, prod) or by the pair rule (max, min).
+// Aggregates combine in FP64 (sum, prod) or by the pair rule (max, min).
 template <int OP> __device__ __forceinline__ ScanRec rec_id()
 {
     if constexpr (OP == NT2G_SCAN_SUM) return ScanRec{0.0, 0.0f, 0};
@@ -317,38 +140,376 @@ template <int OP> __device__ __forceinline__ ScanRec rec_combine(const ScanRec &
     else return to_rec<OP>(SE<OP>::combine(from_rec<OP>(a), from_rec<OP>(b)));
 }
 
-// Phase 2: per segment, replace the chunk aggregates by their exclusive
-// prefixes in order (few chunks: one thread per segment).
-template <int OP>
-__global__ void __launch_bounds__(kScanThreads) k_scan_prefix(ScanRec *__restrict__ rec, int64_t n_seg, int64_t q,
-                                                              int64_t cs)
+// ----------------------------------------- contiguous segments (lo == 1) --
+// Tiles of up to 128 x RUN elements staged in shared memory: whatever the
+// segment's length and alignment, global memory sees whole aligned 16-byte
+// accesses in warp order.  (One-warp tiles, each lane reading 16 consecutive
+// elements straight from global memory, took 156 us for cumsum of 8190 columns
+// of 4099, where every access is 4 bytes and a warp's are 64 bytes apart; this
+// takes 43.)  A thread owns RUN consecutive elements: odd, so the threads read
+// conflict-free from shared memory at any alignment, and many, so that the
+// scan across threads is shared by them (at 17 a thread and 256 threads it was
+// a third of the instructions, 55 us).
+// What bounds it: HBM (6.2 TB/s of the 6.8 a copy reaches), with the issue
+// slots of two compensated adds an element close behind.
+// One pass over long segments, tiles adding up the aggregates that the tiles
+// before them publish, was slower: a tile spends 14 of its 20 us on chip
+// waiting for round trips queued behind the loads of its own SM (93 us for
+// 33.5M elements; fold 30 + scan 44 here).
+
+// Element e (0 <= e < len) of a tile sits at buf[mis + e], mis the tile's
+// offset from a 16-byte boundary, so whole vectors copy without a shift.
+__device__ __forceinline__ int misalign(const float *p) { return (int)(((uintptr_t)p >> 2) & 3); }
+
+__device__ __forceinline__ void tile_fetch(const float *g, int len, float *buf)
 {
-    // record c of segment s at rec[s * ss + c * cs]: ss = q, cs = 1 for contiguous
-    // scans; ss = 1, cs = n_seg (chunk-major, coalesced over segments) for strided ones
-    const int64_t ss = cs == 1 ? q : 1;
+    const int mis = misalign(g), first = (4 - mis) & 3;  // elements before the first whole vector
+    const int nv = len > first ? (len - first) >> 2 : 0, tail = first + 4 * nv;
+    uint32_t to = (uint32_t)__cvta_generic_to_shared(buf + mis + first) + 16 * threadIdx.x;
+    const float *from = g + first + 4 * threadIdx.x;
+#pragma unroll 3
+    for (int v = threadIdx.x; v < nv; v += kLineThreads, to += 16 * kLineThreads, from += 4 * kLineThreads)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to), "l"(from) : "memory");
+    if (threadIdx.x < 4) {  // the ends
+        const int e = tail + (int)threadIdx.x;
+        if ((int)threadIdx.x < first && (int)threadIdx.x < len) buf[mis + threadIdx.x] = g[threadIdx.x];
+        if (e < len) buf[mis + e] = g[e];
+    }
+}
+__device__ __forceinline__ void tile_arrived()
+{
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+}
+
+__device__ __forceinline__ void tile_store(float *g, int len, const float *buf, int mis)
+{
+    if (misalign(g) == mis) {
+        const int first = (4 - mis) & 3, nv = len > first ? (len - first) >> 2 : 0, tail = first + 4 * nv;
+        const float4 *from = (const float4 *)(buf + mis + first) + threadIdx.x;
+        float4 *to = (float4 *)(g + first) + threadIdx.x;
+#pragma unroll 3
+        for (int v = threadIdx.x; v < nv; v += kLineThreads, from += kLineThreads, to += kLineThreads) st_stream(to, *from);
+        if (threadIdx.x < 4) {
+            const int e = tail + (int)threadIdx.x;
+            if ((int)threadIdx.x < first && (int)threadIdx.x < len) g[threadIdx.x] = buf[mis + threadIdx.x];
+            if (e < len) g[e] = buf[mis + e];
+        }
+    } else {  // out sits differently from x: coalesced single elements
+        for (int e = threadIdx.x; e < len; e += kLineThreads) g[e] = buf[mis + e];
+    }
+}
+
+// In-order combine over the block's threads; every thread of warp 0 has the
+// result.  s: one record per warp.
+template <int OP> __device__ __forceinline__ ScanRec block_rec(ScanRec r, ScanRec *s)
+{
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const ScanRec o{__shfl_down_sync(0xffffffffu, r.d, off), __shfl_down_sync(0xffffffffu, r.v, off),
+                        __shfl_down_sync(0xffffffffu, r.h, off)};
+        if ((lane & (2 * off - 1)) == 0) r = rec_combine<OP>(r, o);
+    }
+    if (lane == 0) s[wid] = r;
+    __syncthreads();
+    if (wid == 0) {
+        r = s[0];
+        for (int w = 1; w < kLineThreads / 32; ++w) r = rec_combine<OP>(r, s[w]);
+    }
+    return r;
+}
+
+// WALK: block b scans chunk b % q of segment b / q, tile after tile, from the
+// aggregates of the chunks before it (q = 1: a whole segment).
+// PACK: block b scans `pack` whole short segments, one tile (heads restart).
+template <int OP, bool PACK, int RUN>
+__global__ void __launch_bounds__(kLineThreads) k_scan_line(const float *x, int64_t inner, int64_t hi, int pack,
+                                                            int64_t chunk, int64_t q, const ScanRec *__restrict__ rec,
+                                                            float *out)
+{
+    constexpr int kWarps = kLineThreads / 32, kTile = kLineThreads * RUN;
+    __shared__ __align__(16) float buf[kTile + 4];
+    __shared__ SE<OP> wtot[kWarps], wpre[kWarps];
+    __shared__ ScanRec s_rec[kWarps];
+    __shared__ int whead[kWarps];
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    int64_t begin, end, seg = 0, c = 0;
+    if constexpr (PACK) {
+        const int64_t s0 = (int64_t)blockIdx.x * pack, s1 = s0 + pack < hi ? s0 + pack : hi;
+        begin = s0 * inner;
+        end = s1 * inner;
+    } else {
+        seg = blockIdx.x / q;
+        c = blockIdx.x - seg * q;
+        begin = seg * inner + c * chunk;
+        end = (c + 1) * chunk < inner ? begin + chunk : (seg + 1) * inner;
+    }
+    SE<OP> carry = SE<OP>::id();  // warp 0's
+    for (int64_t t0 = begin; t0 < end; t0 += kTile) {
+        const int len = (int)(end - t0 < kTile ? end - t0 : kTile);
+        const int mis = misalign(x + t0);
+        tile_fetch(x + t0, len, buf);
+        if (!PACK && c > 0 && t0 == begin) {  // the chunks before this one, consecutive ones to a thread
+            const ScanRec *r = rec + seg * q;
+            const int64_t per = (c + kLineThreads - 1) / kLineThreads, i1 = (tid + 1) * per < c ? (tid + 1) * per : c;
+            ScanRec p = rec_id<OP>();
+            for (int64_t i = tid * per; i < i1; ++i) p = rec_combine<OP>(p, r[i]);
+            carry = from_rec<OP>(block_rec<OP>(p, s_rec));
+        }
+        tile_arrived();
+        // PACK: a short tile still occupies every thread.  WALK runs past a
+        // segment's end into whatever the buffer holds: nothing before the end
+        // depends on it.
+        const int per = PACK ? (len + kLineThreads - 1) / kLineThreads | 1 : RUN, i0 = tid * per;
+        const int cnt = len - i0 < per ? (len > i0 ? len - i0 : 0) : per;
+        float *p = buf + mis + i0;
+        const int n32 = (int)inner, r0 = PACK ? i0 % n32 : 1;  // PACK: position in the segment
+        SE<OP> inc = SE<OP>::id();
+        int head = 0;
+        if constexpr (!PACK) {
+#pragma unroll
+            for (int j = 0; j < RUN; ++j) inc.push(p[j]);
+        } else {
+            for (int j = 0, r = r0; j < cnt; ++j) {
+                if (r == 0) { inc = SE<OP>::id(); head = 1; }
+                inc.push(p[j]);
+                if (++r == n32) r = 0;
+            }
+        }
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const SE<OP> o = inc.shfl_up(off);
+            const int oh = PACK ? __shfl_up_sync(0xffffffffu, head, off) : 0;
+            if (lane >= off) {
+                if (!PACK || !head) inc = SE<OP>::combine(o, inc);
+                head |= oh;
+            }
+        }
+        if (lane == 31) {
+            wtot[wid] = inc;
+            whead[wid] = head;
+        }
+        SE<OP> ex = inc.shfl_up(1);
+        int exh = PACK ? __shfl_up_sync(0xffffffffu, head, 1) : 0;
+        if (lane == 0) { ex = SE<OP>::id(); exh = 0; }
+        __syncthreads();
+        if (wid == 0) {  // every warp's prefix, and the next tile's carry
+            SE<OP> pre = SE<OP>::id();
+            for (int w = 0; w < kWarps; ++w) {
+                if (w == lane) pre = carry;
+                carry = PACK && whead[w] ? wtot[w] : SE<OP>::combine(carry, wtot[w]);
+            }
+            if (lane < kWarps) wpre[lane] = pre;
+        }
+        __syncthreads();
+        SE<OP> run = PACK && exh ? ex : SE<OP>::combine(wpre[wid], ex);
+        if constexpr (!PACK) {
+#pragma unroll
+            for (int j = 0; j < RUN; ++j) {
+                run.push(p[j]);
+                p[j] = run.out();
+            }
+        } else {
+            for (int j = 0, r = r0; j < cnt; ++j) {
+                if (r == 0) run = SE<OP>::id();
+                run.push(p[j]);
+                if (++r == n32) r = 0;
+                p[j] = run.out();
+            }
+        }
+        __syncthreads();
+        tile_store(out + t0, len, buf, mis);
+        if (PACK) break;
+        __syncthreads();  // the next tile reuses the buffer
+    }
+}
+
+// The aggregate of chunk b % q of segment b / q.
+template <int OP>
+__global__ void __launch_bounds__(kLineThreads) k_scan_fold(const float *__restrict__ x, int64_t inner, int64_t chunk,
+                                                            int64_t q, ScanRec *__restrict__ rec)
+{
+    __shared__ ScanRec s_rec[kLineThreads / 32];
+    const int64_t seg = blockIdx.x / q, c = blockIdx.x - seg * q;
+    const int64_t begin = seg * inner + c * chunk, end = (c + 1) * chunk < inner ? begin + chunk : (seg + 1) * inner;
+    const int tid = threadIdx.x;
+    SE<OP> acc = SE<OP>::id();
+    if constexpr (OP == NT2G_SCAN_SUM || OP == NT2G_SCAN_PROD) {
+        // the order does not matter to the aggregate: whole vectors, eight loads
+        // in flight a thread, from the chunk's end to its start
+        const int64_t first = begin + ((4 - misalign(x + begin)) & 3), nv = end > first ? (end - first) >> 2 : 0;
+        const float4 *v = (const float4 *)(x + first) + (nv - 1 - tid);
+        int64_t left = nv - tid;
+        constexpr int kBatch = 8 * kLineThreads;
+        if (left > kBatch - kLineThreads) {
+            float4 f[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) f[u] = __ldg(v - u * kLineThreads);
+            while (true) {
+                left -= kBatch;
+                v -= kBatch;
+                const bool more = left > kBatch - kLineThreads;
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    const float4 e = f[u];
+                    if (more) f[u] = __ldg(v - u * kLineThreads);
+                    acc.push(e.x); acc.push(e.y); acc.push(e.z); acc.push(e.w);
+                }
+                if (!more) break;
+            }
+        }
+        for (; left > 0; left -= kLineThreads, v -= kLineThreads) {
+            const float4 f = __ldg(v);
+            acc.push(f.x); acc.push(f.y); acc.push(f.z); acc.push(f.w);
+        }
+        const int64_t e = tid < 4 ? begin + tid : first + 4 * nv + tid - 4;  // the ends
+        if (tid < 4 ? e < first && e < end : tid < 8 && e >= first && e < end) acc.push(x[e]);
+    } else {
+        __shared__ __align__(16) float buf[kTileMax + 4];
+        const int64_t tiles = (end - begin + kTileMax - 1) / kTileMax;
+        for (int64_t t = tiles - 1; t >= 0; --t) {
+            const int64_t t0 = begin + t * kTileMax;
+            const int len = (int)(end - t0 < kTileMax ? end - t0 : kTileMax), mis = misalign(x + t0);
+            tile_fetch(x + t0, len, buf);
+            tile_arrived();
+            const int i0 = tid * kRun, cnt = len - i0 < kRun ? (len > i0 ? len - i0 : 0) : kRun;
+            SE<OP> r = SE<OP>::id();
+#pragma unroll
+            for (int j = 0; j < kRun; ++j)
+                if (j < cnt) r.push(buf[mis + i0 + j]);
+            // thread by thread across tiles would not be in order: the tile first
+            const ScanRec tot = block_rec<OP>(to_rec<OP>(r), s_rec);
+            if (tid == 0) acc = SE<OP>::combine(from_rec<OP>(tot), acc);
+            __syncthreads();
+        }
+        if (tid == 0) rec[blockIdx.x] = to_rec<OP>(acc);
+        return;
+    }
+    const ScanRec tot = block_rec<OP>(to_rec<OP>(acc), s_rec);
+    if (tid == 0) rec[blockIdx.x] = tot;
+}
+
+// ---------------------------------------------- strided scans (lo > 1) --
+// Thread per segment (VEC: four neighbouring segments via float4) over the
+// chunk [c*ck, min((c+1)*ck, inner)) of the scan range; grid.y = chunk.
+// FOLD: the chunk's aggregate.  Else the scan, from the aggregates of the chunks above (`prefixes`: k_scan_prefix* has
+// replaced them by their sums).
+template <int OP, int VEC, bool FOLD>
+__global__ void __launch_bounds__(kScanThreads) k_scan_outer(const float *x, int64_t lo, int64_t inner, int64_t hi,
+                                                             int64_t ck, int64_t q, bool prefixes,
+                                                             ScanRec *__restrict__ rec, float *out)
+{
+    const int64_t lv = lo / VEC, n_seg = lo * hi;
+    const int64_t c = blockIdx.y;
+    const int64_t k0 = c * ck, k1 = (k0 + ck < inner) ? k0 + ck : inner;
+    // groups of kGroup rows: all loads of a group are issued before its scan
+    constexpr int kGroup = (OP == NT2G_SCAN_PROD && VEC == 4) ? 4 : VEC == 4 ? 8 : 16;
+    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < lv * hi; t += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t h = t / lv, l = (t - h * lv) * VEC;
+        const int64_t base = l + lo * inner * h;
+        SE<OP> carry[VEC];
+#pragma unroll
+        for (int v = 0; v < VEC; ++v) {
+            const int64_t seg = l + v + lo * h;
+            if (FOLD || q == 1 || c == 0) {
+                carry[v] = SE<OP>::id();
+            } else if (prefixes) {
+                carry[v] = from_rec<OP>(rec[c * n_seg + seg]);
+            } else {
+                ScanRec p = rec[seg];
+                for (int64_t i = 1; i < c; ++i) p = rec_combine<OP>(p, rec[i * n_seg + seg]);
+                carry[v] = from_rec<OP>(p);
+            }
+        }
+        auto fetch = [&](const float *p, float (&e)[VEC]) {
+            if constexpr (VEC == 4) {
+                const float4 f = FOLD ? __ldg((const float4 *)p) : ld_stream((const float4 *)p);
+                e[0] = f.x; e[1] = f.y; e[2] = f.z; e[3] = f.w;
+            } else {
+                e[0] = FOLD ? __ldg(p) : ld_stream(p);
+            }
+        };
+        if constexpr (FOLD) {
+            const float *p = x + base + lo * k0;
+            int64_t k = k1 - k0;
+            for (; k >= kGroup; k -= kGroup) {
+                float e[kGroup][VEC];
+#pragma unroll
+                for (int g = 0; g < kGroup; ++g, p += lo) fetch(p, e[g]);
+#pragma unroll
+                for (int g = 0; g < kGroup; ++g)
+#pragma unroll
+                    for (int v = 0; v < VEC; ++v) carry[v].push(e[g][v]);
+            }
+            for (; k > 0; --k, p += lo) {
+                float e[VEC];
+                fetch(p, e);
+#pragma unroll
+                for (int v = 0; v < VEC; ++v) carry[v].push(e[v]);
+            }
+#pragma unroll
+            for (int v = 0; v < VEC; ++v) rec[c * n_seg + (l + v + lo * h)] = to_rec<OP>(carry[v]);
+        } else {
+            const float *p = x + base + lo * k0;
+            float *o = out + base + lo * k0;
+            auto step = [&](const float (&e)[VEC]) {
+                float r[VEC];
+#pragma unroll
+                for (int v = 0; v < VEC; ++v) {
+                    carry[v].push(e[v]);
+                    r[v] = carry[v].out();
+                }
+                if constexpr (VEC == 4) st_stream((float4 *)o, make_float4(r[0], r[1], r[2], r[3]));
+                else st_stream(o, r[0]);
+                o += lo;
+            };
+            int64_t k = k1 - k0;
+            for (; k >= kGroup; k -= kGroup) {
+                float e[kGroup][VEC];
+#pragma unroll
+                for (int g = 0; g < kGroup; ++g, p += lo) fetch(p, e[g]);
+#pragma unroll
+                for (int g = 0; g < kGroup; ++g) step(e[g]);
+            }
+            for (; k > 0; --k, p += lo) {
+                float e[VEC];
+                fetch(p, e);
+                step(e);
+            }
+        }
+    }
+}
+
+// Strided scans of many chunks: per segment, the chunk aggregates replaced by
+// their exclusive prefixes in order (one thread per segment).
+template <int OP>
+__global__ void __launch_bounds__(kScanThreads) k_scan_prefix(ScanRec *__restrict__ rec, int64_t n_seg, int64_t q)
+{
+    // record c of segment s at rec[s + c * n_seg]: coalesced over segments
     for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < n_seg; s += (int64_t)gridDim.x * blockDim.x) {
-        ScanRec *r = rec + s * ss;
+        ScanRec *r = rec + s;
         ScanRec acc = rec_id<OP>();
         int64_t c = 0;
         for (; c + 8 <= q; c += 8) {  // eight independent loads in flight
             ScanRec a[8];
 #pragma unroll
-            for (int u = 0; u < 8; ++u) a[u] = r[(c + u) * cs];
+            for (int u = 0; u < 8; ++u) a[u] = r[(c + u) * n_seg];
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
-                r[(c + u) * cs] = acc;
+                r[(c + u) * n_seg] = acc;
                 acc = rec_combine<OP>(acc, a[u]);
             }
         }
         for (; c < q; ++c) {
-            const ScanRec a = r[c * cs];
-            r[c * cs] = acc;
+            const ScanRec a = r[c * n_seg];
+            r[c * n_seg] = acc;
             acc = rec_combine<OP>(acc, a);
         }
     }
 }
 
-// Phase 2 for many chunks: one block per segment (below).  The combine order
+// For more chunks still: one block per segment.  The combine order
 // is fixed for a given q.
 template <int OP> __device__ __forceinline__ ScanRec rec_shfl_up(const ScanRec &a, int off)
 {
@@ -358,7 +519,7 @@ template <int OP> __device__ __forceinline__ ScanRec rec_shfl_up(const ScanRec &
 
 template <int OP>
 __global__ void __launch_bounds__(kScanThreads) k_scan_prefix_block(ScanRec *__restrict__ rec, int64_t n_seg,
-                                                                    int64_t q, int64_t cs)
+                                                                    int64_t q)
 {
     // tiles of kScanThreads x 8 consecutive records: each thread loads its 8
     // (independent loads), the thread totals are scanned in order across the
@@ -368,13 +529,13 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_prefix_block(ScanRec *__r
     __shared__ ScanRec carry_s;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     for (int64_t s = blockIdx.x; s < n_seg; s += gridDim.x) {
-        ScanRec *r = rec + s * (cs == 1 ? q : 1);
+        ScanRec *r = rec + s;
         ScanRec carry = rec_id<OP>();
         for (int64_t t0 = 0; t0 < q; t0 += (int64_t)kScanThreads * kPer) {
             const int64_t c0 = t0 + (int64_t)tid * kPer;
             ScanRec a[kPer];
 #pragma unroll
-            for (int u = 0; u < kPer; ++u) a[u] = c0 + u < q ? r[(c0 + u) * cs] : rec_id<OP>();
+            for (int u = 0; u < kPer; ++u) a[u] = c0 + u < q ? r[(c0 + u) * n_seg] : rec_id<OP>();
             ScanRec tot = rec_id<OP>();
 #pragma unroll
             for (int u = 0; u < kPer; ++u) tot = rec_combine<OP>(tot, a[u]);
@@ -401,7 +562,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_prefix_block(ScanRec *__r
             ScanRec pre = rec_combine<OP>(wtot[wid], ex);
 #pragma unroll
             for (int u = 0; u < kPer; ++u) {
-                if (c0 + u < q) r[(c0 + u) * cs] = pre;
+                if (c0 + u < q) r[(c0 + u) * n_seg] = pre;
                 pre = rec_combine<OP>(pre, a[u]);
             }
             carry = carry_s;
@@ -432,30 +593,36 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_nt2(const float *x, int64
 
 // ---------------------------------------------------------------- plans --
 struct ScanPlan {
-    int kind = 1;  // 1 contiguous, 2 strided
-    int vec = 0;
-    int64_t chunk = 0, q = 1;
+    bool lines = false;        // contiguous segments
+    int pack = 1;              // lines: short segments per block
+    int vec = 1;               // strided: segments per thread
+    int64_t chunk = 0, q = 1;  // elements per chunk, chunks per segment
 };
 
+// Contiguous: segments shorter than kPackBelow share a block's tile, as many
+// as still leave 13 blocks to each SM; longer ones get a block each, which is
+// one pass, when they are one tile or fill the GPU; else chunks of whole
+// tiles, 12 blocks to each SM (one wave: 13 fit).  Strided: a thread per
+// segment (four with float4) if that gives 1024 threads to each SM, else
+// chunks of at least 16 rows.
 static ScanPlan plan_scan(int64_t lo, int64_t inner, int64_t hi, bool aligned)
 {
     ScanPlan p;
     if (lo == 1) {
-        p.kind = 1;
-        p.vec = aligned && inner % 4 == 0;
-        const int64_t want = 152 * 8 * 4;
-        int64_t chunk = kScanChunk;
-        if (hi * ((inner + chunk - 1) / chunk) < want) {
-            const int64_t per = (want + hi - 1) / hi;
-            chunk = (inner + per - 1) / per;
-            if (chunk < 1024) chunk = 1024;
+        p.lines = true;
+        p.chunk = inner;
+        if (inner < kPackBelow) {
+            const int64_t most = kTileMax / (inner > 0 ? inner : 1), spread = (hi + 152 * 13 - 1) / (152 * 13);
+            p.pack = (int)(most < spread ? most : spread);
+        } else if (inner > kTileMax && hi < kLineChunks) {
+            const int64_t tiles = (inner + kTileMax - 1) / kTileMax;
+            const int64_t per = (hi * tiles + kLineChunks - 1) / kLineChunks;  // tiles per chunk
+            p.q = (tiles + per - 1) / per;
+            p.chunk = (tiles + p.q - 1) / p.q * kTileMax;
+            p.q = (inner + p.chunk - 1) / p.chunk;
         }
-        chunk = (chunk + 511) / 512 * 512;
-        p.chunk = chunk;
-        p.q = inner > 0 ? (inner + chunk - 1) / chunk : 1;
         return p;
     }
-    p.kind = 2;
     p.vec = aligned && lo % 4 == 0 ? 4 : 1;
     const int64_t threads = lo * hi / p.vec;
     int64_t q = 1;
@@ -470,19 +637,34 @@ static ScanPlan plan_scan(int64_t lo, int64_t inner, int64_t hi, bool aligned)
     return p;
 }
 
+// Contiguous scans need less than they ask for: 16 bytes for each of the
+// 4864 chunks of at most 16384 elements that one warp each once took.
 nt2g_status scan_workspace_bytes(int64_t lo, int64_t inner, int64_t hi, size_t *bytes)
 {
-    const ScanPlan a = plan_scan(lo, inner, hi, true), b = plan_scan(lo, inner, hi, false);
-    const int64_t q = a.q > b.q ? a.q : b.q;
+    int64_t q;
+    if (lo == 1) {
+        const int64_t want = 152 * 8 * 4;
+        int64_t chunk = 16384;
+        if (hi * ((inner + chunk - 1) / chunk) < want) {
+            const int64_t per = hi > 0 ? (want + hi - 1) / hi : 1;
+            chunk = (inner + per - 1) / per;
+            if (chunk < 1024) chunk = 1024;
+        }
+        chunk = (chunk + 511) / 512 * 512;
+        q = inner > 0 ? (inner + chunk - 1) / chunk : 1;
+    } else {
+        const ScanPlan a = plan_scan(lo, inner, hi, true), b = plan_scan(lo, inner, hi, false);
+        q = a.q > b.q ? a.q : b.q;
+    }
     *bytes = q > 1 ? (size_t)(lo * hi) * (size_t)q * sizeof(ScanRec) : 0;
     return NT2G_OK;
 }
 
-template <int OP> static void launch_prefix(ScanRec *rec, int64_t n_seg, int64_t q, int64_t cs, cudaStream_t st)
+template <int OP> static void launch_prefix(ScanRec *rec, int64_t n_seg, int64_t q, cudaStream_t st)
 {
     auto cap = [](int64_t g) { return (int)(g < 152 * 32 ? (g > 0 ? g : 1) : 152 * 32); };
-    if (q >= 512) k_scan_prefix_block<OP><<<cap(n_seg), kScanThreads, 0, st>>>(rec, n_seg, q, cs);
-    else k_scan_prefix<OP><<<cap((n_seg + kScanThreads - 1) / kScanThreads), kScanThreads, 0, st>>>(rec, n_seg, q, cs);
+    if (q >= 512) k_scan_prefix_block<OP><<<cap(n_seg), kScanThreads, 0, st>>>(rec, n_seg, q);
+    else k_scan_prefix<OP><<<cap((n_seg + kScanThreads - 1) / kScanThreads), kScanThreads, 0, st>>>(rec, n_seg, q);
 }
 
 template <int OP>
@@ -502,28 +684,36 @@ static nt2g_status launch_scan_op(const float *x, int64_t lo, int64_t inner, int
         return NT2G_ERR_INVALID;
     }
     ScanRec *rec = (ScanRec *)ws;
-    if (p.kind == 1) {
-        const int grid = cap((hi * p.q + 7) / 8);
-        if (p.q > 1) {
-            k_scan_inner<OP, 1><<<grid, kScanThreads, 0, st>>>(x, inner, hi, p.chunk, p.q, p.vec, rec, out);
-            launch_prefix<OP>(rec, n_seg, p.q, 1, st);
+    if (p.lines) {
+        // a launch takes up to 2^30 blocks
+        const int64_t most = ((int64_t)1 << 30) / p.q * p.pack;
+        for (int64_t s0 = 0; s0 < hi; s0 += most) {
+            const int64_t n = hi - s0 < most ? hi - s0 : most;
+            const unsigned g = (unsigned)((n + p.pack - 1) / p.pack * p.q);
+            const float *xs = x + s0 * inner;
+            float *os = out + s0 * inner;
+            if (p.q > 1) k_scan_fold<OP><<<g, kLineThreads, 0, st>>>(xs, inner, p.chunk, p.q, rec);
+#define NT2G_LINE(PACK, RUN) k_scan_line<OP, PACK, RUN><<<g, kLineThreads, 0, st>>>(xs, inner, n, p.pack, p.chunk, p.q, \
+                                                                                    rec, os)
+            if (p.pack > 1) NT2G_LINE(true, kRun);
+            else if (p.chunk <= kLineThreads * 9) NT2G_LINE(false, 9);
+            else if (p.chunk <= kLineThreads * 17) NT2G_LINE(false, 17);
+            else NT2G_LINE(false, kRun);
+#undef NT2G_LINE
         }
-        k_scan_inner<OP, 3><<<grid, kScanThreads, 0, st>>>(x, inner, hi, p.chunk, p.q, p.vec, rec, out);
     } else {
-        dim3 grid(cap((n_seg / p.vec + kScanThreads - 1) / kScanThreads), (unsigned)p.q);
-        if (p.vec == 4) {
-            if (p.q > 1) {
-                k_scan_outer<OP, 4, 1><<<grid, kScanThreads, 0, st>>>(x, lo, inner, hi, p.chunk, p.q, rec, out);
-                launch_prefix<OP>(rec, n_seg, p.q, n_seg, st);
-            }
-            k_scan_outer<OP, 4, 3><<<grid, kScanThreads, 0, st>>>(x, lo, inner, hi, p.chunk, p.q, rec, out);
-        } else {
-            if (p.q > 1) {
-                k_scan_outer<OP, 1, 1><<<grid, kScanThreads, 0, st>>>(x, lo, inner, hi, p.chunk, p.q, rec, out);
-                launch_prefix<OP>(rec, n_seg, p.q, n_seg, st);
-            }
-            k_scan_outer<OP, 1, 3><<<grid, kScanThreads, 0, st>>>(x, lo, inner, hi, p.chunk, p.q, rec, out);
+        const dim3 grid(cap((n_seg / p.vec + kScanThreads - 1) / kScanThreads), (unsigned)p.q);
+        const bool prefixes = p.q > kInlinePrefix;
+#define NT2G_OUTER(VEC, FOLD) k_scan_outer<OP, VEC, FOLD><<<grid, kScanThreads, 0, st>>>(x, lo, inner, hi, p.chunk, p.q, \
+                                                                                         prefixes, rec, out)
+        if (p.q > 1) {
+            if (p.vec == 4) NT2G_OUTER(4, true);
+            else NT2G_OUTER(1, true);
+            if (prefixes) launch_prefix<OP>(rec, n_seg, p.q, st);
         }
+        if (p.vec == 4) NT2G_OUTER(4, false);
+        else NT2G_OUTER(1, false);
+#undef NT2G_OUTER
     }
     NT2G_LAUNCH_CHECK("scan launch");
     return NT2G_OK;
