@@ -31,24 +31,25 @@ static_assert((int)SUM == (int)NT2G_FOLD_SUM &&
               "fold op numbering");
 
 constexpr int kFoldThreads = kThreads;
-constexpr int64_t kChunk = 16384;        // elements per warp work item (contiguous folds)
-constexpr int64_t kSmallSeg = 64;        // segments up to this length: one thread each
-constexpr int64_t kTargetThreads = 152 * 1024;
+constexpr int64_t kChunk = 16384;        // elements per chunk a contiguous fold asks workspace for
+constexpr int64_t kBlocks = 152 * 12;    // blocks a fold is cut into at least: a few waves, so that none is nearly empty
+constexpr int64_t kSmallSeg = 64;        // (many) segments up to this length: one thread each
 
 // A table as a fold source: streaming loads.
 struct RawSrc {
+    static constexpr int kBatch = 4;  // vectors a thread has in flight
     const float *x;
     __device__ __forceinline__ float at(int64_t pos) const { return ld_stream(x + pos); }
     __device__ __forceinline__ float4 at4(int64_t pos) const { return ld_stream((const float4 *)(x + pos)); }
 };
 
-template <int OP, bool FINAL, bool IDX>
-__global__ void __launch_bounds__(kFoldThreads) k_fold_inner(RawSrc src, int64_t inner, int64_t hi, int64_t chunk,
+template <int OP, bool FINAL, bool IDX, int G>
+__global__ void __launch_bounds__(kFoldThreads, is_var(OP) ? 3 : 4) k_fold_inner(RawSrc src, int64_t inner, int64_t hi, int64_t chunk,
                                                              int64_t q, int vec, Partial *__restrict__ part,
                                                              float *__restrict__ out, int64_t *__restrict__ index,
                                                              const float *__restrict__ cen, double *__restrict__ out64)
 {
-    inner_body<RawSrc, OP, FINAL, IDX>(src, inner, hi, chunk, q, vec, part, out, index, cen, out64);
+    inner_body<RawSrc, OP, FINAL, IDX, G>(src, inner, hi, chunk, q, vec, part, out, index, cen, out64);
 }
 
 template <int OP>
@@ -60,7 +61,7 @@ __global__ void __launch_bounds__(kFoldThreads) k_fold_short(RawSrc src, int64_t
 }
 
 template <int OP, int VEC, bool FINAL>
-__global__ void __launch_bounds__(kFoldThreads) k_fold_outer(RawSrc src, int64_t lo, int64_t inner, int64_t hi,
+__global__ void __launch_bounds__(kFoldThreads, is_var(OP) ? 3 : 4) k_fold_outer(RawSrc src, int64_t lo, int64_t inner, int64_t hi,
                                                              int64_t ck, int64_t q, Partial *__restrict__ part,
                                                              float *__restrict__ out, int64_t *__restrict__ index,
                                                              const float *__restrict__ cen, double *__restrict__ out64)
@@ -76,127 +77,152 @@ __global__ void __launch_bounds__(kFoldThreads) k_fold_nt2(RawSrc src, int64_t l
     nt2_body<RawSrc, OP>(src, lo, inner, hi, out, index, cen);
 }
 
-// Combine the q partials of each output in order.
+// Combine the q partials of each output: 32 outputs a block, the partials of
+// neighbouring outputs next to each other, in eight consecutive ranges of
+// chunks (a thread each), whose totals then combine in order.
+constexpr int kRanges = kFoldThreads / 32;
 template <int OP>
 __global__ void __launch_bounds__(kFoldThreads) k_fold_finish(const Partial *__restrict__ part, int64_t n_out,
-                                                              int64_t q, int64_t inner, float *__restrict__ out,
-                                                              int64_t *__restrict__ index, const float *__restrict__ cen,
-                                                              double *__restrict__ out64)
+                                                              int64_t q, int64_t chunk, int64_t inner,
+                                                              float *__restrict__ out, int64_t *__restrict__ index,
+                                                              const float *__restrict__ cen, double *__restrict__ out64)
 {
-    for (int64_t o = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; o < n_out; o += (int64_t)gridDim.x * blockDim.x) {
-        const Partial *p = part + o * q;
-        if (is_sum(OP) || OP == PROD) {
-            double t = OP == PROD ? 1.0 : 0.0;
-            for (int64_t c = 0; c < q; ++c) t = OP == PROD ? t * p[c].d : t + p[c].d;
-            fold_put<OP>(out, out64, o, n_out, t, inner, cen);
-        } else {
-            Best b{0.0f, -1, -1};
-            for (int64_t c = 0; c < q; ++c)
-                if (p[c].b.ilast >= 0) b = b.ilast < 0 ? p[c].b : best_merge<OP == MAX>(b, p[c].b);
-            out[o] = b.v;
-            if (index) index[o] = b.ifirst;
+    __shared__ Total<OP> st[kRanges][32];
+    const int lane = threadIdx.x & 31, range = threadIdx.x >> 5;
+    const int64_t per = (q + kRanges - 1) / kRanges, c0 = range * per, c1 = c0 + per < q ? c0 + per : q;
+    for (int64_t o0 = (int64_t)blockIdx.x * 32; o0 < n_out; o0 += (int64_t)gridDim.x * 32) {
+        const int64_t o = o0 + lane;
+        Total<OP> t;
+        if (o < n_out)
+#pragma unroll 4
+            for (int64_t c = c0; c < c1; ++c)
+                t.add(part[c * n_out + o], (double)(inner - c * chunk < chunk ? inner - c * chunk : chunk));
+        st[range][lane] = t;
+        __syncthreads();
+        if (range == 0 && o < n_out) {
+            for (int r = 1; r < kRanges; ++r) {
+                const int64_t k0 = r * per * chunk, k1 = (r + 1) * per * chunk < inner ? (r + 1) * per * chunk : inner;
+                t.add(st[r][lane], k1 > k0 ? (double)(k1 - k0) : 0.0);
+            }
+            t.put(out, index, out64, o, n_out, inner, cen);
         }
+        __syncthreads();
     }
 }
 
-// Many partials per output (global folds): one block per output, thread t
-// combining partials t, t+T, t+2T, ... in that order, then a fixed
-// shared-memory tree over the threads' results.  Deterministic for a given q.
+// Few outputs of many partials (global folds): one block per output, thread t
+// combining its consecutive partials, then a shared-memory tree over the
+// threads' totals in order.
 template <int OP>
 __global__ void __launch_bounds__(kFoldThreads) k_fold_finish_block(const Partial *__restrict__ part, int64_t n_out,
-                                                                    int64_t q, int64_t inner, float *__restrict__ out,
+                                                                    int64_t q, int64_t chunk, int64_t inner,
+                                                                    float *__restrict__ out,
                                                                     int64_t *__restrict__ index,
                                                                     const float *__restrict__ cen,
                                                                     double *__restrict__ out64)
 {
-    constexpr bool DBL = is_sum(OP) || OP == PROD;
-    __shared__ double sd[kFoldThreads];
-    __shared__ Best sb[kFoldThreads];
+    __shared__ Total<OP> st[kFoldThreads];
+    const int64_t per = (q + kFoldThreads - 1) / kFoldThreads, c0 = threadIdx.x * per,
+                  c1 = c0 + per < q ? c0 + per : q;
     for (int64_t o = blockIdx.x; o < n_out; o += gridDim.x) {
-        const Partial *p = part + o * q;
-        if (DBL) {
-            double t = OP == PROD ? 1.0 : 0.0;
-#pragma unroll 4
-            for (int64_t c = threadIdx.x; c < q; c += blockDim.x) t = OP == PROD ? t * p[c].d : t + p[c].d;
-            sd[threadIdx.x] = t;
-        } else {
-            Best b{0.0f, -1, -1};
-#pragma unroll 4
-            for (int64_t c = threadIdx.x; c < q; c += blockDim.x) b = best_merge<OP == MAX>(b, p[c].b);
-            sb[threadIdx.x] = b;
-        }
+        Total<OP> t;
+#pragma unroll 8
+        for (int64_t c = c0; c < c1; ++c)
+            t.add(part[c * n_out + o], (double)(inner - c * chunk < chunk ? inner - c * chunk : chunk));
+        st[threadIdx.x] = t;
         __syncthreads();
-        for (int w = kFoldThreads / 2; w > 0; w >>= 1) {
-            if ((int)threadIdx.x < w) {
-                if (DBL) sd[threadIdx.x] = OP == PROD ? sd[threadIdx.x] * sd[threadIdx.x + w]
-                                                      : sd[threadIdx.x] + sd[threadIdx.x + w];
-                else sb[threadIdx.x] = best_merge<OP == MAX>(sb[threadIdx.x], sb[threadIdx.x + w]);
+        for (int w = 1; w < kFoldThreads; w <<= 1) {
+            if ((threadIdx.x & (2 * w - 1)) == 0) {
+                const int64_t k0 = (threadIdx.x + w) * per * chunk, k = k0 + w * per * chunk, k1 = k < inner ? k : inner;
+                st[threadIdx.x].add(st[threadIdx.x + w], k1 > k0 ? (double)(k1 - k0) : 0.0);
             }
             __syncthreads();
         }
-        if (threadIdx.x == 0) {
-            if (DBL) {
-                fold_put<OP>(out, out64, o, n_out, sd[0], inner, cen);
-            } else {
-                out[o] = sb[0].v;
-                if (index) index[o] = sb[0].ifirst;
-            }
-        }
+        if (threadIdx.x == 0) st[0].put(out, index, out64, o, n_out, inner, cen);
         __syncthreads();
     }
 }
 
 // --------------------------------------------------------------- plans --
 struct FoldPlan {
-    int kind = 0;       // 0 short segments, 1 warp chunks (lo == 1), 2 strided
+    int kind = 0;       // 0 short segments, 1 contiguous (lo == 1), 2 strided
+    int group = 0;      // contiguous: log2 of the threads per segment, as the index 0: 8, 1: 32, 2: 256
     int64_t chunk = 0;  // elements per chunk along the fold
     int64_t q = 1;      // chunks per output
     int vec = 0;
 };
 
-static FoldPlan plan_fold(int64_t lo, int64_t inner, int64_t hi, bool aligned)
+static FoldPlan plan_fold(int64_t lo, int64_t inner, int64_t hi, bool aligned, int op)
 {
     FoldPlan p;
     if (lo == 1) {
         if (inner <= kSmallSeg && hi >= 1024) { p.kind = 0; return p; }
         p.kind = 1;
-        p.vec = aligned && (inner % 4 == 0);
-        // enough warp items to fill the GPU: 8 warps per SM at least 4 times over
-        const int64_t want = 152 * 8 * 4;
-        int64_t chunk = kChunk;
-        if (hi * ((inner + chunk - 1) / chunk) < want) {
-            int64_t per = (want + hi - 1) / hi;
-            chunk = (inner + per - 1) / per;
-            if (chunk < 1024) chunk = 1024;
+        p.vec = aligned;
+        // at least 32 elements (eight float4 loads) a thread, with more threads a
+        // segment where there are too few segments to fill the GPU
+        p.group = inner <= 256 ? 0 : 1;
+        if (p.group == 0 && inner > 64 && hi < 152 * 32) p.group = 1;
+        if (p.group == 1 && inner > 512 && hi < (inner <= 2048 ? 152 * 8 : 152 * 24)) p.group = 2;
+        p.chunk = inner > 0 ? inner : 1;
+        if (p.group == 2 && hi < kBlocks) {
+            const int64_t per = (kBlocks + hi - 1) / hi;
+            int64_t chunk = (inner + per - 1) / per;
+            if (chunk < 4096) chunk = 4096;
+            p.chunk = (chunk + 1023) / 1024 * 1024;
+            p.q = (inner + p.chunk - 1) / p.chunk;
+            if (p.q < 1) p.q = 1;
         }
-        chunk = (chunk + 127) / 128 * 128;
-        p.chunk = chunk;
-        p.q = (inner + chunk - 1) / chunk;
         return p;
     }
     p.kind = 2;
     p.vec = aligned && (lo % 4 == 0) ? 4 : 1;
-    const int64_t threads = lo * hi / p.vec;
-    int64_t q = 1;
-    if (threads < kTargetThreads) {
-        q = (kTargetThreads + threads - 1) / threads;
-        const int64_t qmax = inner / 16 > 0 ? inner / 16 : 1;
-        if (q > qmax) q = qmax;
-        if (q > 65535) q = 65535;  // grid.y
-    }
+    const int64_t columns = (lo * hi / p.vec + 31) / 32;  // blocks side by side
+    // (a variance's partials cost some twenty FP64 instructions each to combine)
+    int64_t q = ((is_var(op) ? kBlocks / 2 : kBlocks) + columns - 1) / columns;
+    const int64_t qmax = inner / 64 > 0 ? inner / 64 : 1;  // eight rows a warp at least
+    if (q > qmax) q = qmax;
+    if (q > 65535) q = 65535;  // grid.y
     if ((inner + q - 1) / q > (1 << 30)) q = (inner + (1 << 30) - 1) >> 30;  // 32-bit positions in a chunk
     p.chunk = (inner + q - 1) / q;
     p.q = (inner + p.chunk - 1) / p.chunk;
     return p;
 }
 
-// Workspace: the partials of the chunked plans, then (for var/stdev) each
-// output's centre and its rounding error, 16-byte aligned.
+// Workspace: the partials of the chunked plans, then (for two-pass folds) each
+// output's centre and its rounding error, 16-byte aligned.  A fold asks for
+// room for a partial of every warp (contiguous) or every 1024 threads an SM
+// (strided); the plans above, a partial per block, need less.
+static int64_t fold_chunks_asked(int64_t lo, int64_t inner, int64_t hi, bool aligned)
+{
+    if (lo == 1) {
+        if (inner <= 64 && hi >= 1024) return 1;
+        const int64_t want = 152 * 8 * 4;
+        int64_t chunk = kChunk;
+        if (hi * ((inner + chunk - 1) / chunk) < want) {
+            const int64_t per = hi > 0 ? (want + hi - 1) / hi : 1;
+            chunk = (inner + per - 1) / per;
+            if (chunk < 1024) chunk = 1024;
+        }
+        chunk = (chunk + 127) / 128 * 128;
+        return (inner + chunk - 1) / chunk;
+    }
+    const int64_t threads = lo * hi / (aligned && (lo % 4 == 0) ? 4 : 1);
+    int64_t q = 1;
+    if (threads > 0 && threads < 152 * 1024) {
+        q = (152 * 1024 + threads - 1) / threads;
+        const int64_t qmax = inner / 16 > 0 ? inner / 16 : 1;
+        if (q > qmax) q = qmax;
+        if (q > 65535) q = 65535;
+    }
+    if ((inner + q - 1) / q > (1 << 30)) q = (inner + (1 << 30) - 1) >> 30;
+    const int64_t chunk = (inner + q - 1) / q;
+    return chunk > 0 ? (inner + chunk - 1) / chunk : 1;
+}
 static size_t fold_partial_bytes(int64_t lo, int64_t inner, int64_t hi)
 {
-    FoldPlan p = plan_fold(lo, inner, hi, true);
-    FoldPlan u = plan_fold(lo, inner, hi, false);
-    int64_t q = p.q > u.q ? p.q : u.q;
+    const int64_t a = fold_chunks_asked(lo, inner, hi, true), b = fold_chunks_asked(lo, inner, hi, false);
+    const int64_t q = a > b ? a : b;
     return q > 1 ? (size_t)(lo * hi) * (size_t)q * sizeof(Partial) : 0;
 }
 static size_t fold_centre_offset(int64_t lo, int64_t inner, int64_t hi)
@@ -242,13 +268,16 @@ static nt2g_status launch_fold_op(const FoldInput &in, int64_t lo, int64_t inner
     const int precision = in.precision;
     const int64_t n_out = lo * hi;
     if constexpr (is_two_pass(OP)) {
-        if (!cen) {  // first the centre of every output: NT2's float mean, or (fast) the mean and its rounding
-                     // error; for nanmean the count of non-NaN elements
+        // (a variance asks for the centres' room under either policy)
+        if (!cen && (!ws || fold_centre_offset(lo, inner, hi) + (size_t)n_out * 2 * sizeof(float) > ws_bytes)) {
+            set_error("fold: workspace of %zu bytes, %zu needed", ws_bytes,
+                      fold_centre_offset(lo, inner, hi) + (size_t)n_out * 2 * sizeof(float));
+            return NT2G_ERR_INVALID;
+        }
+        // first the centre of every output: NT2's float mean, or (fast, meanad) the mean and its rounding
+        // error; for nanmean the count of non-NaN elements
+        if (!cen && (is_two_pass_fast(OP) || precision == NT2G_PREC_NT2 || inner == 0)) {
             const size_t off = fold_centre_offset(lo, inner, hi);
-            if (!ws || off + (size_t)n_out * 2 * sizeof(float) > ws_bytes) {
-                set_error("fold: workspace of %zu bytes, %zu needed", ws_bytes, off + (size_t)n_out * 2 * sizeof(float));
-                return NT2G_ERR_INVALID;
-            }
             float *c = (float *)((char *)ws + off);
             nt2g_status s;
             if constexpr (OP == NANMEAN)
@@ -286,7 +315,7 @@ static nt2g_status launch_fold_op(const FoldInput &in, int64_t lo, int64_t inner
         if (ce != cudaSuccess) return cuda_status(ce, "fold launch");
         return NT2G_OK;
     }
-    FoldPlan p = plan_fold(lo, inner, hi, in.aligned);
+    FoldPlan p = plan_fold(lo, inner, hi, in.aligned, OP);
     if (p.q > 1 && (size_t)(n_out * p.q) * sizeof(Partial) > ws_bytes) {
         set_error("fold: workspace of %zu bytes, %zu needed", ws_bytes, (size_t)(n_out * p.q) * sizeof(Partial));
         return NT2G_ERR_INVALID;
@@ -303,25 +332,35 @@ static nt2g_status launch_fold_op(const FoldInput &in, int64_t lo, int64_t inner
         }
     } else if (p.kind == 1) {
         const int64_t items = hi * p.q;
-        const dim3 g(cap((items + 7) / 8));
+        static const int kItemsPerBlock[3] = {kFoldThreads / 8, kFoldThreads / 32, 1};
+        // several items a block, which shares the FP64 of their results, while
+        // that leaves enough blocks for a few waves
+        int64_t per = kItemsPerBlock[p.group];
+        while (p.q == 1 && per < kItems && (items + 2 * per - 1) / (2 * per) >= kBlocks) per *= 2;
+        const dim3 g((unsigned)((items + per - 1) / per));
         const bool idx = index != nullptr && (OP == MAX || OP == MIN);
         const bool fin = p.q == 1;
         int64_t chunk = p.chunk, q = p.q;
         int vec = p.vec;
         if (!in.expr) {
-#define NT2G_INNER(F, I) k_fold_inner<OP, F, I><<<g, kFoldThreads, 0, st>>>(src, inner, hi, chunk, q, vec, part, out, \
-                                                                            index, cen, out64)
-            if (fin) { if (idx) NT2G_INNER(true, true); else NT2G_INNER(true, false); }
-            else { if (idx) NT2G_INNER(false, true); else NT2G_INNER(false, false); }
+#define NT2G_INNER(F, I, G) k_fold_inner<OP, F, I, G><<<g, kFoldThreads, 0, st>>>(src, inner, hi, chunk, q, vec, part, out, \
+                                                                               index, cen, out64)
+#define NT2G_INNER_I(F, G) do { if (EXT && idx) NT2G_INNER(F, EXT, G); else NT2G_INNER(F, false, G); } while (0)
+            constexpr bool EXT = OP == MAX || OP == MIN;  // only these have positions
+            if (!fin) NT2G_INNER_I(false, 256);
+            else if (p.group == 0) NT2G_INNER_I(true, 8);
+            else if (p.group == 1) NT2G_INNER_I(true, 32);
+            else NT2G_INNER_I(true, 256);
+#undef NT2G_INNER_I
 #undef NT2G_INNER
             ce = cudaGetLastError();
         } else {
             void *pr[] = {(void *)jargs, &inner, &hi, &chunk, &q, &vec, &part, &out, &index, &cen, &out64};
-            ce = launch_by_handle(jk->inner[fin][idx], g, pr, st);
+            ce = launch_by_handle(jk->inner[fin ? p.group : 3][idx], g, pr, st);
         }
     } else {
         const int64_t threads = n_out / p.vec;
-        const dim3 g(cap((threads + kFoldThreads - 1) / kFoldThreads), (unsigned)p.q);
+        const dim3 g(cap((threads + 31) / 32), (unsigned)p.q);
         const bool fin = p.q == 1;
         int64_t chunk = p.chunk, q = p.q;
         if (!in.expr) {
@@ -338,11 +377,13 @@ static nt2g_status launch_fold_op(const FoldInput &in, int64_t lo, int64_t inner
     }
     if (ce != cudaSuccess) return cuda_status(ce, "fold launch");
     if (p.q > 1 && p.kind != 0) {
-        if (p.q >= 512)
-            k_fold_finish_block<OP><<<cap(n_out), kFoldThreads, 0, st>>>(part, n_out, p.q, inner, out, index, cen, out64);
+        // a block per output where eight threads each would walk long ranges
+        if (n_out < 32 || (n_out <= 2048 && p.q > 128))
+            k_fold_finish_block<OP><<<cap(n_out), kFoldThreads, 0, st>>>(part, n_out, p.q, p.chunk, inner, out, index, cen,
+                                                                        out64);
         else
-            k_fold_finish<OP><<<cap((n_out + kFoldThreads - 1) / kFoldThreads), kFoldThreads, 0, st>>>(
-                part, n_out, p.q, inner, out, index, cen, out64);
+            k_fold_finish<OP><<<cap((n_out + 31) / 32), kFoldThreads, 0, st>>>(
+                part, n_out, p.q, p.chunk, inner, out, index, cen, out64);
         NT2G_LAUNCH_CHECK("fold combine launch");
     }
     return NT2G_OK;

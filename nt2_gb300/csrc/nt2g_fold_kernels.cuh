@@ -34,14 +34,17 @@
 // pass, then the centred sum of squares.
 //
 // Fast policy: sums are compensated FP32 (TwoSum; squares carry their FMA
-// product error) per chunk, chunks combined in FP64 in index order; var/stdev
-// centre on the float mean and correct for its rounding error
-// (sum (x - m)^2 - n (mu - m)^2, mu the FP64 mean); prod in FP64; max/min are
-// exact.  Contiguous segments are cut into chunks, one warp per chunk with
-// 128-bit loads; strided folds run one thread per output (four with 128-bit
-// loads) over chunks of the fold range.  With more than one chunk per output,
-// partials go to the caller's workspace and a second kernel combines them in
-// order, so results are deterministic for a given shape.
+// product error) per thread, chunks combined in FP64; var/stdev take one pass:
+// the deviations from an element of the chunk, and their squares, are summed
+// compensated, and chunks combine by their means in FP64 (a pivot among the
+// data keeps the correction to the mean at most n times the result); meanad
+// centres on the mean of a first pass; prod in FP64; max/min are exact.
+// Contiguous segments are folded by 8, 32 or 256 threads each (inner_body),
+// strided ones by warps over 32 columns (four each with 128-bit loads), rows
+// split over a block's warps (outer_body), so that a block hands on one
+// partial per output.  With more than one chunk per output, partials go to
+// the caller's workspace and a second kernel combines them in a fixed order,
+// so results are deterministic for a given shape.
 #pragma once
 #if !defined(__CUDACC_RTC__)
 #include <stdint.h>
@@ -66,14 +69,17 @@ enum : int {
 };
 
 constexpr int kThreads = 256;
+constexpr int kItems = 64;  // work items of a block of inner_body, at most
 
 __host__ __device__ constexpr bool is_var(int op) { return op == VAR || op == STDEV || op == VAR1 || op == STDEV1; }
 // counts of elements: nbtrue and the logical folds all/any/none over x != 0
 __host__ __device__ constexpr bool is_count(int op) { return op == NBTRUE || op == ALL || op == ANY || op == NONE; }
 // folds of the deviations from each output's mean
 __host__ __device__ constexpr bool is_centred(int op) { return is_var(op) || op == MEANAD; }
-// folds that need a per-output value from a first pass (the centre, the count)
+// folds that need a per-output value from a first pass (the centre, the count);
+// the fast policy takes variances in one
 __host__ __device__ constexpr bool is_two_pass(int op) { return is_centred(op) || op == NANMEAN; }
+__host__ __device__ constexpr bool is_two_pass_fast(int op) { return op == MEANAD || op == NANMEAN; }
 __host__ __device__ constexpr bool is_sum(int op)
 {
     return op == SUM || op == MEAN || op == ASUM1 || op == ASUM2 || op == NORM2 || op == MEAN_C || is_var(op) ||
@@ -154,11 +160,9 @@ template <int OP> __device__ __forceinline__ void sum_elem(CSum &a, float x)
     }
 }
 
-// variance terms: (x - m)^2 with the difference kept exactly as dh + dl
-// (TwoSum) and the square's rounding error carried, so the sum of squared
-// deviations is compensated like the other sums.  Mean absolute deviation
-// terms: |x - mu| with mu = m + md (the float mean and its rounding error),
-// as |dh| plus the low part dl - md with the sign of dh (|lo| where dh is 0).
+// Mean absolute deviation terms: |x - mu| with mu = m + md (the float mean and
+// its rounding error), the difference kept exactly as dh + dl (TwoSum), as
+// |dh| plus the low part dl - md with the sign of dh (|lo| where dh is 0).
 template <int OP> __device__ __forceinline__ void sum_elem_c(CSum &a, float x, float m, float md = 0.0f)
 {
     if constexpr (OP == MEANAD) {
@@ -168,23 +172,71 @@ template <int OP> __device__ __forceinline__ void sum_elem_c(CSum &a, float x, f
         const float lo = __fsub_rn(dl, md);
         csum_add(a, fabsf(dh));
         a.c = __fadd_rn(a.c, dh > 0.0f ? lo : dh < 0.0f ? -lo : fabsf(lo));
-    } else if constexpr (is_var(OP)) {
-        const float dh = __fsub_rn(x, m);
-        const float bb = __fsub_rn(dh, x);
-        const float dl = __fadd_rn(__fsub_rn(x, __fsub_rn(dh, bb)), __fsub_rn(-m, bb));
-        const float p = __fmul_rn(dh, dh);
-        csum_add(a, p);
-        a.c = __fadd_rn(a.c, __fmaf_rn(2.0f * dh, dl, __fmaf_rn(dh, dh, -p)));
     } else {
         sum_elem<OP>(a, x);
     }
 }
 
 // ---------------------------------------------------------------- partials --
-// 32 bytes per (output, chunk): a double (sums, prod) or a Best.
+// Per (chunk, output), chunk-major: a compensated sum (sums; variances: of the
+// deviations from the chunk's pivot, and of their squares), a product or a
+// Best.  Turned into FP64 only where many outputs or chunks are at hand at
+// once: an FP64 instruction takes a warp sixteen cycles, however few of its
+// lanes need it.
+struct Sums {
+    CSum s1, s2;
+    float piv;
+};
 struct Partial {
-    double d;
-    Best b;
+    union {
+        Sums v;
+        double d;
+        Best b;
+    };
+};
+
+// Chunks of one output combined in order.  A variance's sums are shifted to
+// the first chunk's pivot in FP64: what cancels when they are brought to the
+// mean is at most the number of elements times the result, 2^-53 of that.
+template <int OP> struct Total {
+    double t = OP == PROD ? 1.0 : 0.0, t2 = 0.0, p0 = 0.0;
+    Best b{0.0f, -1, -1};
+    bool any = false;
+    __device__ __forceinline__ void add(const Partial &p, double n)
+    {
+        if constexpr (is_var(OP)) {
+            const double s1 = (double)p.v.s1.s + (double)p.v.s1.c, s2 = (double)p.v.s2.s + (double)p.v.s2.c;
+            if (!any) p0 = (double)p.v.piv;
+            const double d = (double)p.v.piv - p0, nd = n * d;
+            t += s1 + nd;
+            t2 += s2 + d * (2.0 * s1 + nd);
+            any = true;
+        } else if constexpr (is_sum(OP)) {
+            t += (double)p.v.s1.s + (double)p.v.s1.c;
+        } else if constexpr (OP == PROD) {
+            t *= p.d;
+        } else {
+            b = best_merge<OP == MAX>(b, p.b);
+        }
+    }
+    __device__ __forceinline__ void add(const Total &o, double n)  // n: the elements of o
+    {
+        if constexpr (is_var(OP)) {
+            if (!o.any) return;
+            if (!any) { *this = o; return; }
+            const double d = o.p0 - p0, nd = n * d;
+            t += o.t + nd;
+            t2 += o.t2 + d * (2.0 * o.t + nd);
+        } else if constexpr (is_sum(OP)) {
+            t += o.t;
+        } else if constexpr (OP == PROD) {
+            t *= o.t;
+        } else {
+            b = best_merge<OP == MAX>(b, o.b);
+        }
+    }
+    __device__ __forceinline__ void put(float *out, int64_t *index, double *out64, int64_t o, int64_t n_out, int64_t inner,
+                                        const float *cen) const;
 };
 
 // The FP64 value of a sum-type (or product) fold before it is rounded to the
@@ -199,9 +251,9 @@ template <int OP> __device__ __forceinline__ double finish_double(double t, int6
 // Writes output o of a sum-type (or product) fold from its FP64 total (and,
 // when out64 is given, that total's FP64 result: the mean, the norm, the
 // variance, ... before rounding to float).
-// Variance: the sum of squares about the float centre m, corrected to the
-// exact mean mu = m + delta (sum (x - m)^2 = sum (x - mu)^2 + n delta^2),
-// divided by n - 1 (by n for VAR1/STDEV1; 1 when n <= 1).
+// Variance: t is the sum of squares about the mean, divided by n - 1 (by n for
+// VAR1/STDEV1; 1 when n <= 1); not a number (an infinity or a NaN among the
+// elements, or their squares past the float range) gives 0.
 template <int OP>
 __device__ __forceinline__ void fold_put(float *out, double *out64, int64_t o, int64_t n_out, double t, int64_t inner,
                                          const float *cen)
@@ -220,10 +272,8 @@ __device__ __forceinline__ void fold_put(float *out, double *out64, int64_t o, i
         const double c = (double)cen[o];
         r = t / (c > 1.0 ? c : 1.0);
     } else if constexpr (is_var(OP)) {
-        const double d = (double)cen[n_out + o];
         const double n = (double)inner;
-        double v = t - n * d * d;
-        v = v > 0.0 ? v : 0.0;
+        double v = t > 0.0 ? t : 0.0;
         const bool by_n = OP == VAR1 || OP == STDEV1;
         if (inner > 1) v /= by_n ? n : n - 1.0;
         r = (OP == STDEV || OP == STDEV1) ? sqrt(v) : v;
@@ -234,82 +284,405 @@ __device__ __forceinline__ void fold_put(float *out, double *out64, int64_t o, i
     if (out64) out64[o] = r;
 }
 
-// ------------------------------------------- warp-shuffle merges (fast) --
-__device__ __forceinline__ double warp_prod(double a)
+template <int OP>
+__device__ __forceinline__ void Total<OP>::put(float *out, int64_t *index, double *out64, int64_t o, int64_t n_out,
+                                               int64_t inner, const float *cen) const
+{
+    if constexpr (is_var(OP)) {
+        fold_put<OP>(out, out64, o, n_out, t2 - t * (t / (double)inner), inner, cen);
+    } else if constexpr (is_sum(OP) || OP == PROD) {
+        fold_put<OP>(out, out64, o, n_out, t, inner, cen);
+    } else {
+        out[o] = b.v;
+        if (index) index[o] = b.ifirst;
+    }
+}
+
+// ------------------------------------------------- per-thread accumulators --
+// One-pass variance: the sums of the deviations d = x - p from a pivot p and of
+// their squares, both compensated, d exact as dh + dl (TwoSum) and the square's
+// rounding error carried; two elements per packed f32x2 instruction (each half
+// rounds as the scalar operation does), which halves the issue slots of its 28
+// operations an element pair.
+struct VarAcc {
+    typedef unsigned long long F2;
+    F2 s1, c1, s2, c2, p;
+    static __device__ __forceinline__ F2 pack(float a, float b)
+    {
+        F2 r;
+        asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+        return r;
+    }
+    static __device__ __forceinline__ float half(F2 v, int i)
+    {
+        float a, b;
+        asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+        return i ? b : a;
+    }
+    static __device__ __forceinline__ F2 add(F2 a, F2 b)
+    {
+        F2 r;
+        asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+        return r;
+    }
+    static __device__ __forceinline__ F2 sub(F2 a, F2 b)
+    {
+        F2 r;
+        asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+        return r;
+    }
+    static __device__ __forceinline__ F2 mul(F2 a, F2 b)
+    {
+        F2 r;
+        asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+        return r;
+    }
+    static __device__ __forceinline__ F2 fma(F2 a, F2 b, F2 c)
+    {
+        F2 r;
+        asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+        return r;
+    }
+    static __device__ __forceinline__ void csum2(F2 &s, F2 &c, F2 v)
+    {
+        const F2 t = add(s, v), bb = sub(t, s);
+        c = add(c, add(sub(s, sub(t, bb)), sub(v, bb)));
+        s = t;
+    }
+    __device__ __forceinline__ void start(float pivot, float pivot1)
+    {
+        s1 = c1 = s2 = c2 = pack(0.0f, 0.0f);
+        p = pack(pivot, pivot1);
+    }
+    __device__ __forceinline__ void take2(F2 x)
+    {
+        const F2 d = sub(x, p), nd = sub(p, x);
+        const F2 bb = sub(d, x);  // TwoSum of x and -p: bb is -p's share
+        const F2 dl = sub(sub(x, sub(d, bb)), add(p, bb));
+        const F2 q = mul(d, d);
+        csum2(s1, c1, d);
+        c1 = add(c1, dl);
+        csum2(s2, c2, q);
+        c2 = sub(c2, fma(add(nd, nd), dl, fma(nd, d, q)));  // less q - d^2 - 2 d dl
+    }
+    // one element: the other half adds zero
+    __device__ __forceinline__ void take(float x) { take2(pack(x, half(p, 1))); }
+    __device__ __forceinline__ Sums sums() const
+    {
+        Sums r{CSum{half(s1, 0), half(c1, 0)}, CSum{half(s2, 0), half(c2, 0)}, half(p, 0)};
+        csum_merge(r.s1, CSum{half(s1, 1), half(c1, 1)});
+        csum_merge(r.s2, CSum{half(s2, 1), half(c2, 1)});
+        return r;
+    }
+    // Squares past the float range though no element is infinite or not a
+    // number: the pivot may be far off, the mean is worth a second try.
+    static __device__ __forceinline__ bool over(const Sums &r)
+    {
+        const float a = r.s1.s + r.s1.c, b = r.s2.s + r.s2.c;
+        return a - a == 0.0f && b - b != 0.0f;
+    }
+    static __device__ __forceinline__ float mean(const Sums &r, int64_t n)
+    {
+        return r.piv + (r.s1.s + r.s1.c) / (float)n;
+    }
+};
+
+// max/min over batches of up to 32 elements: the batch's extreme over the W
+// lanes that work together first (an instruction an element), and only when
+// it reaches the running one are the positions looked for -- about the
+// logarithm of the number of batches for data in no order.  W lanes of `mask`
+// call it together.
+__device__ __forceinline__ float max_nan(float a, float b)
+{
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float min_nan(float a, float b)
+{
+    float r;
+    asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+template <bool MX, bool FIRST, int W> struct BatchRun {
+    float cur = MX ? -NT2G_FOLD_INF : NT2G_FOLD_INF, v = 0.0f;
+    int32_t ifirst = -1, ilast = -1, inan = -1;
+    // elements e[u][c], u < n, at positions pos + u * step + c
+    template <int U, int V>
+    __device__ __forceinline__ void batch(const float (&e)[U][V], int n, int32_t pos, int32_t step, unsigned mask)
+    {
+        float m = MX ? -NT2G_FOLD_INF : NT2G_FOLD_INF;
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+            for (int c = 0; c < V; ++c)
+                if (u < n) m = MX ? max_nan(m, e[u][c]) : min_nan(m, e[u][c]);
+        if constexpr (W > 1) {
+#pragma unroll
+            for (int off = W / 2; off; off >>= 1) {
+                const float o = __shfl_xor_sync(mask, m, off);
+                m = MX ? max_nan(m, o) : min_nan(m, o);
+            }
+        }
+        if (better<MX>(cur, m)) return;
+        // Equal numbers have equal bits but for zeros, so only there does the last
+        // one matter; otherwise the first position of a new extreme is all.
+        if (better<MX>(m, cur)) {
+            cur = v = m;
+            ifirst = ilast = -1;
+            if (!FIRST && m != 0.0f) {
+                ilast = pos;
+            } else if (m != 0.0f) {
+#pragma unroll
+                for (int u = U - 1; u >= 0; --u)
+#pragma unroll
+                    for (int c = V - 1; c >= 0; --c)
+                        if (u < n && e[u][c] == m) ifirst = pos + u * step + c;
+                ilast = ifirst;
+            }
+        } else if (U * V == 1 && n && e[0][0] == m && m != 0.0f) {  // the ends of a segment come last
+            ifirst = (unsigned)pos < (unsigned)ifirst ? pos : ifirst;
+            ilast = ifirst;
+        }
+        if (m != m) rare<true>(e, n, pos, step);  // elements beside a NaN count for nothing: the result is the NaN
+        else if (m == 0.0f) rare<false>(e, n, pos, step);
+    }
+    // The first NaN, or the first and the last zero.
+    template <bool NANS, int U, int V>
+    __device__ __forceinline__ void rare(const float (&e)[U][V], int n, int32_t pos, int32_t step)
+    {
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+            for (int c = 0; c < V; ++c)
+                if (u < n && (NANS ? e[u][c] != e[u][c] : e[u][c] == 0.0f)) {
+                    const int32_t at = pos + u * step + c;
+                    if (NANS) {
+                        inan = (unsigned)at < (unsigned)inan ? at : inan;
+                    } else {
+                        ifirst = (unsigned)at < (unsigned)ifirst ? at : ifirst;
+                        if (at > ilast) { ilast = at; v = e[u][c]; }
+                    }
+                }
+    }
+    // The result of the W lanes together (they share `cur`).
+    __device__ __forceinline__ Best best(int64_t base, unsigned mask) const
+    {
+        const unsigned nan = lanes_min((unsigned)inan, mask), first = lanes_min((unsigned)ifirst, mask);
+        const unsigned last = ~lanes_min(~(unsigned)(ilast + 1), mask);  // the largest ilast + 1
+        const int owner = __ffs(__ballot_sync(mask, ilast >= 0 && (unsigned)(ilast + 1) == last) & mask) - 1;
+        const float val = __shfl_sync(mask, v, owner < 0 ? (int)(threadIdx.x & 31) : owner);
+        if (nan != ~0u) return Best{__int_as_float(0x7fffffff), base + nan, base + nan};
+        if (last == 0) return Best{0.0f, -1, -1};
+        return Best{val, base + last - 1, FIRST ? base + first : base + last - 1};
+    }
+    static __device__ __forceinline__ unsigned lanes_min(unsigned x, unsigned mask)
+    {
+        if constexpr (W == 32) {
+            return __reduce_min_sync(mask, x);
+        } else {
+#pragma unroll
+            for (int off = W / 2; off; off >>= 1) {
+                const unsigned o = __shfl_xor_sync(mask, x, off);
+                x = o < x ? o : x;
+            }
+            return x;
+        }
+    }
+    __device__ __forceinline__ Best to_best(int64_t base) const
+    {
+        if (inan >= 0) return Best{__int_as_float(0x7fffffff), base + inan, base + inan};
+        if (ilast < 0) return Best{0.0f, -1, -1};
+        return Best{v, base + ilast, base + ifirst};
+    }
+};
+
+// ------------------------------------------- merges over W lanes (fast) --
+template <int W> __device__ __forceinline__ CSum lanes_csum(CSum a, unsigned mask)
 {
 #pragma unroll
-    for (int off = 16; off; off >>= 1) a *= __shfl_down_sync(0xffffffffu, a, off);
+    for (int off = W / 2; off; off >>= 1) {
+        const CSum b{__shfl_down_sync(mask, a.s, off), __shfl_down_sync(mask, a.c, off)};
+        csum_merge(a, b);
+    }
     return a;
 }
-template <bool MX> __device__ __forceinline__ Best warp_best(Best a)
+template <int W> __device__ __forceinline__ double lanes_prod(double a, unsigned mask)
 {
 #pragma unroll
-    for (int off = 16; off; off >>= 1) {
-        Best b{__shfl_down_sync(0xffffffffu, a.v, off), __shfl_down_sync(0xffffffffu, a.ilast, off),
-               __shfl_down_sync(0xffffffffu, a.ifirst, off)};
+    for (int off = W / 2; off; off >>= 1) a *= __shfl_down_sync(mask, a, off);
+    return a;
+}
+template <bool MX, int W> __device__ __forceinline__ Best lanes_best(Best a, unsigned mask)
+{
+#pragma unroll
+    for (int off = W / 2; off; off >>= 1) {
+        const Best b{__shfl_down_sync(mask, a.v, off), __shfl_down_sync(mask, a.ilast, off),
+                     __shfl_down_sync(mask, a.ifirst, off)};
         a = best_merge<MX>(a, b);  // symmetric: lanes hold interleaved elements
     }
     return a;
 }
 
 // ----------------------------------------- contiguous segments (lo == 1) --
-// One warp per (segment, chunk) work item.  FINAL: one chunk per segment, the
-// warp writes the output directly.  vec: segment starts and chunk bounds are
-// multiples of 4 and the source is 16-byte addressable.
-template <class Src, int OP, bool FINAL, bool IDX>
+// G threads (8, 32 or the block's 256) per (segment, chunk) work item, a few
+// items a block one after the other: a segment's loads are in flight at once
+// and blocks are short (a warp per segment of 6000 left the last wave of
+// blocks alone on the GPU for a quarter of the time: 39 us for 8192 of them,
+// 33 now).  Whole vectors wherever the segment starts: the ends before the
+// first and after the last multiple of 4 go element by element.  FINAL: one
+// chunk per segment; a block turns all its items into outputs at its end, a
+// thread each (FP64).  vec: the source is 16-byte addressable at multiples of 4.
+template <class Src, int OP, bool FINAL, bool IDX, int G>
 __device__ __forceinline__ void inner_body(const Src &src, int64_t inner, int64_t hi, int64_t chunk, int64_t q,
                                            int vec, Partial *__restrict__ part, float *__restrict__ out,
                                            int64_t *__restrict__ index, const float *__restrict__ cen,
                                            double *__restrict__ out64)
 {
-    const int lane = threadIdx.x & 31;
-    const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t item = warp; item < hi * q; item += nwarps) {
-        const int64_t seg = item / q, c = item - seg * q;
+    constexpr bool MX = OP == MAX, EXT = OP == MAX || OP == MIN;
+    constexpr int W = G < 32 ? G : 32, kGroups = kThreads / G, kWarps = kThreads / 32;
+    constexpr int kBatch = Src::kBatch;
+    __shared__ Partial s_item[FINAL ? kItems : 1];
+    __shared__ Partial s_warp[2][kWarps];
+    __shared__ float s_mean;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, tid = threadIdx.x % G;
+    const unsigned mask = W == 32 ? 0xffffffffu : 0xffu << (lane & 24);
+    const int64_t items = hi * q;
+    const int per = (int)(((items + gridDim.x - 1) / gridDim.x + kGroups - 1) / kGroups) * kGroups;  // <= kItems
+    const int64_t item0 = (int64_t)blockIdx.x * per;
+    int turn = 0;
+    for (int i = threadIdx.x / G; i < per && item0 + i < items; i += kGroups) {
+        const int64_t item = item0 + i, seg = item / q, c = item - seg * q;
         const int64_t k0 = c * chunk, k1 = (k0 + chunk < inner) ? k0 + chunk : inner;
-        const int64_t base = seg * inner;
+        const int64_t p0 = seg * inner + k0, p1 = seg * inner + k1;  // positions in the table
         CSum acc{0.0f, 0.0f};
         double prod = 1.0;
-        const float m = is_centred(OP) ? cen[seg] : 0.0f;
+        VarAcc var;
+        BatchRun<MX, IDX, W> run;
+        const float m = OP == MEANAD ? cen[seg] : 0.0f;
         const float md = OP == MEANAD ? cen[hi + seg] : 0.0f;
-        Run<OP == MAX, IDX> run[4];  // one per float4 component: four independent chains
-        auto take = [&](int cc, float v, int32_t k) {  // k: position relative to k0
-            if (is_sum(OP)) sum_elem_c<OP>(acc, v, m, md);
-            else if (OP == PROD) prod *= (double)v;
-            else run[cc].add(v, k);
-        };
-        int64_t k = k0;
-        if (vec) {
-            const int64_t v1 = k1 >> 2;
-#pragma unroll 8
-            for (int64_t j = (k0 >> 2) + lane; j < v1; j += 32) {
-                const float4 f = src.at4(base + 4 * j);
-                const int32_t r0 = (int32_t)(4 * j - k0);
-                take(0, f.x, r0); take(1, f.y, r0 + 1); take(2, f.z, r0 + 2); take(3, f.w, r0 + 3);
-            }
-            k = v1 << 2;
-        }
-        for (int64_t j = k + lane; j < k1; j += 32) take(0, src.at(base + j), (int32_t)(j - k0));
-        Partial r;
-        if (is_sum(OP)) {
-            acc = warp_csum(acc);
-            r.d = (double)acc.s + (double)acc.c;
-        } else if (OP == PROD) {
-            r.d = warp_prod(prod);
-        } else {
-            constexpr bool MX = OP == MAX;
-            Best b = best_merge<MX>(best_merge<MX>(run[0].to_best(k0), run[1].to_best(k0)),
-                                    best_merge<MX>(run[2].to_best(k0), run[3].to_best(k0)));
-            r.b = warp_best<MX>(b);
-        }
-        if (lane == 0) {
-            if (FINAL) {
-                if (is_sum(OP) || OP == PROD) fold_put<OP>(out, out64, seg, hi, r.d, inner, cen);
-                else { out[seg] = r.b.v; if (index) index[seg] = r.b.ifirst; }
+        // n batch rows e[u][0..V) at position pos + u * step (relative to p0)
+        auto take = [&](const auto &e, int n, int32_t pos, int32_t step) {
+            [[maybe_unused]] constexpr int U = sizeof(e) / sizeof(e[0]), V = sizeof(e[0]) / sizeof(float);
+            if constexpr (EXT) {
+                run.batch(e, n, pos, step, mask);
             } else {
-                part[item] = r;
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    if (u >= n) break;
+                    if constexpr (is_var(OP) && V == 4) {
+                        var.take2(VarAcc::pack(e[u][0], e[u][1]));
+                        var.take2(VarAcc::pack(e[u][2], e[u][3]));
+                    } else {
+#pragma unroll
+                        for (int v = 0; v < V; ++v) {
+                            if constexpr (is_var(OP)) var.take(e[u][v]);
+                            else if constexpr (OP == PROD) prod *= (double)e[u][v];
+                            else sum_elem_c<OP>(acc, e[u][v], m, md);
+                        }
+                    }
+                }
             }
+        };
+        auto sweep = [&]() {
+            if (vec) {
+                const int64_t a = (p0 + 3) >> 2, b = p1 >> 2;  // whole vectors [a, b)
+                for (int64_t j = a; j < b; j += kBatch * G) {
+                    const int64_t left = b - j - tid;
+                    float e[kBatch][4];
+                    const int n = left <= 0 ? 0 : left > (kBatch - 1) * G ? kBatch : (int)((left + G - 1) / G);
+#pragma unroll
+                    for (int u = 0; u < kBatch; ++u) {  // (past the end: the last one again, so that no load waits for a branch)
+                        const int64_t at = j + tid + u * G;
+                        const float4 f = src.at4(4 * (at < b ? at : b - 1));
+                        e[u][0] = f.x; e[u][1] = f.y; e[u][2] = f.z; e[u][3] = f.w;
+                    }
+                    const int32_t pos = (int32_t)(4 * (j + tid) - p0);
+                    if (j + kBatch * G <= b) take(e, kBatch, pos, 4 * G);
+                    else take(e, n, pos, 4 * G);
+                }
+                // up to three elements on either side
+                const int64_t first = 4 * a < p1 ? 4 * a : p1, last = 4 * b > first ? 4 * b : first;
+                if (p0 < first || last < p1) {
+                    const int64_t at = tid < 4 ? p0 + tid : last + tid - 4;
+                    const int n = tid < 4 ? at < first : tid < 8 && at < p1;
+                    float e[1][1];
+                    if (n) e[0][0] = src.at(at);
+                    take(e, n, (int32_t)(at - p0), 0);
+                }
+            } else {
+                for (int64_t j = p0; j < p1; j += kBatch * G) {
+                    const int64_t left = p1 - j - tid;
+                    float e[kBatch][1];
+                    const int n = left <= 0 ? 0 : left > (kBatch - 1) * G ? kBatch : (int)((left + G - 1) / G);
+#pragma unroll
+                    for (int u = 0; u < kBatch; ++u) {
+                        const int64_t at = j + tid + u * G;
+                        e[u][0] = src.at(at < p1 ? at : p1 - 1);
+                    }
+                    take(e, n, (int32_t)(j + tid - p0), G);
+                }
+            }
+        };
+        // the item's threads together; thread 0 of the item has the result.
+        // (Two sets of shared slots in turn: a barrier an item is enough.)
+        Partial r;
+        auto together = [&]() {
+            if constexpr (is_var(OP)) {
+                r.v = var.sums();
+                r.v.s1 = lanes_csum<W>(r.v.s1, mask);
+                r.v.s2 = lanes_csum<W>(r.v.s2, mask);
+            } else if constexpr (is_sum(OP)) {
+                r.v.s1 = lanes_csum<W>(acc, mask);
+            } else if constexpr (OP == PROD) {
+                r.d = lanes_prod<W>(prod, mask);
+            } else {
+                r.b = run.best(k0, mask);
+            }
+            if constexpr (G > 32) {
+                if (lane == 0) s_warp[turn][wid] = r;
+                __syncthreads();
+                if (threadIdx.x < kWarps) {
+                    r = s_warp[turn][lane];
+                    constexpr unsigned few = (1u << kWarps) - 1;
+                    if constexpr (is_sum(OP)) r.v.s1 = lanes_csum<kWarps>(r.v.s1, few);
+                    if constexpr (is_var(OP)) r.v.s2 = lanes_csum<kWarps>(r.v.s2, few);
+                    if constexpr (OP == PROD) r.d = lanes_prod<kWarps>(r.d, few);
+                    if constexpr (EXT) r.b = lanes_best<MX, kWarps>(r.b, few);
+                }
+                turn ^= 1;
+            }
+        };
+        const float piv = is_var(OP) ? src.at(p0) : 0.0f;
+        if constexpr (is_var(OP)) var.start(piv, piv);
+        sweep();
+        together();
+        if constexpr (is_var(OP)) {
+            float mean = VarAcc::over(r.v) ? VarAcc::mean(r.v, k1 - k0) : piv;
+            if constexpr (G > 32) {
+                if (threadIdx.x == 0) s_mean = mean;
+                __syncthreads();
+                mean = s_mean;
+            } else {
+                mean = __shfl_sync(mask, mean, lane & ~(W - 1));
+            }
+            if (mean != piv && mean == mean) {
+                var.start(mean, mean);
+                sweep();
+                together();
+            }
+        }
+        if (tid == 0) {
+            if (FINAL) s_item[i] = r;
+            else part[c * hi + seg] = r;
+        }
+    }
+    if constexpr (FINAL) {
+        __syncthreads();
+        for (int i = threadIdx.x; i < per && item0 + i < items; i += kThreads) {
+            Total<OP> t;
+            t.add(s_item[i], (double)inner);
+            t.put(out, index, out64, item0 + i, hi, inner, cen);
         }
     }
 }
@@ -326,15 +699,30 @@ __device__ __forceinline__ void short_body(const Src &src, int64_t inner, int64_
         CSum acc{0.0f, 0.0f};
         double prod = 1.0;
         Run<OP == MAX> run;
-        const float m = is_centred(OP) ? cen[seg] : 0.0f;
+        VarAcc var;
+        if (is_var(OP)) var.start(src.at(base), src.at(base));
+        const float m = OP == MEANAD ? cen[seg] : 0.0f;
         const float md = OP == MEANAD ? cen[hi + seg] : 0.0f;
         for (int64_t k = 0; k < inner; ++k) {
             const float v = src.at(base + k);
-            if (is_sum(OP)) sum_elem_c<OP>(acc, v, m, md);
+            if (is_var(OP)) var.take(v);
+            else if (is_sum(OP)) sum_elem_c<OP>(acc, v, m, md);
             else if (OP == PROD) prod *= (double)v;
             else run.add(v, (int32_t)k);
         }
-        if (is_sum(OP)) fold_put<OP>(out, out64, seg, hi, (double)acc.s + (double)acc.c, inner, cen);
+        if (is_var(OP)) {
+            Partial r;
+            r.v = var.sums();
+            if (VarAcc::over(r.v)) {
+                const float mean = VarAcc::mean(r.v, inner);
+                var.start(mean, mean);
+                for (int64_t k = 0; k < inner; ++k) var.take(src.at(base + k));
+                r.v = var.sums();
+            }
+            Total<OP> t;
+            t.add(r, (double)inner);
+            t.put(out, index, out64, seg, hi, inner, cen);
+        } else if (is_sum(OP)) fold_put<OP>(out, out64, seg, hi, (double)acc.s + (double)acc.c, inner, cen);
         else if (OP == PROD) { out[seg] = (float)prod; if (out64) out64[seg] = prod; }
         else {
             const Best b = run.to_best(0);
@@ -345,61 +733,161 @@ __device__ __forceinline__ void short_body(const Src &src, int64_t inner, int64_
 }
 
 // ---------------------------------------------- strided folds (lo > 1) --
-// Thread per output (VEC: four consecutive outputs via float4), over the
-// chunk [c*ck, min((c+1)*ck, inner)) of the fold range; grid.y = chunk.
+// A block takes 32 threads' worth of outputs (VEC: four neighbouring ones each,
+// via float4) over the chunk [c*ck, min((c+1)*ck, inner)) of the fold range,
+// grid.y = chunk; its warps take every eighth row, a batch of rows in
+// flight each, and their accumulators combine in shared memory: one partial
+// per output and block.  (A thread per output and chunk wrote eight times the
+// partials -- 20 MB for 6000 rows of 8192, 16 to 49 us to combine -- and had
+// one or two loads in flight.)
 template <class Src, int OP, int VEC, bool FINAL>
 __device__ __forceinline__ void outer_body(const Src &src, int64_t lo, int64_t inner, int64_t hi, int64_t ck,
                                            int64_t q, Partial *__restrict__ part, float *__restrict__ out,
                                            int64_t *__restrict__ index, const float *__restrict__ cen,
                                            double *__restrict__ out64)
 {
+    constexpr bool MX = OP == MAX, EXT = OP == MAX || OP == MIN;
+    constexpr int kWarps = kThreads / 32, kRows = Src::kBatch;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int64_t lv = lo / VEC;  // thread columns per h
     const int64_t c = blockIdx.y;
     const int64_t k0 = c * ck, k1 = (k0 + ck < inner) ? k0 + ck : inner;
-    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < lv * hi; t += (int64_t)gridDim.x * blockDim.x) {
+    for (int64_t t0 = (int64_t)blockIdx.x * 32; t0 < lv * hi; t0 += (int64_t)gridDim.x * 32) {
+        const int64_t t = t0 + lane;
+        const bool live = t < lv * hi;
         const int64_t h = t / lv, l = (t - h * lv) * VEC;
         const int64_t base = l + lo * inner * h;
         CSum acc[VEC];
         double prod[VEC];
-        Run<OP == MAX> run[VEC];
-        float m[VEC], md[VEC];
+        BatchRun<MX, true, 1> run[VEC];
+        // a variance's two sums of each output, one half of VarAcc's pairs each
+        VarAcc var[(VEC + 1) / 2];
+        float m[VEC], md[VEC], piv[VEC];
+        auto start = [&]() {
 #pragma unroll
-        for (int v = 0; v < VEC; ++v) {
-            acc[v] = CSum{0.0f, 0.0f};
-            prod[v] = 1.0;
-            m[v] = is_centred(OP) ? cen[l + v + lo * h] : 0.0f;
-            md[v] = OP == MEANAD ? cen[lo * hi + l + v + lo * h] : 0.0f;
-        }
-        for (int64_t k = k0; k < k1; ++k) {
-            float e[VEC];
+            for (int v = 0; v < VEC; v += 2) var[v / 2].start(piv[v], piv[v + (VEC > 1)]);
+        };
+        auto load = [&](int64_t k, float (&e)[VEC]) {
             if constexpr (VEC == 4) {
                 const float4 f = src.at4(base + lo * k);
                 e[0] = f.x; e[1] = f.y; e[2] = f.z; e[3] = f.w;
             } else {
                 e[0] = src.at(base + lo * k);
             }
+        };
+        // rows k, k + kWarps, ...
+        auto take = [&](const auto &e, int64_t k) {
+            constexpr int U = sizeof(e) / sizeof(e[0]);
+            if constexpr (EXT) {
 #pragma unroll
-            for (int v = 0; v < VEC; ++v) {
-                if (is_sum(OP)) sum_elem_c<OP>(acc[v], e[v], m[v], md[v]);
-                else if (OP == PROD) prod[v] *= (double)e[v];
-                else run[v].add(e[v], (int32_t)(k - k0));
+                for (int v = 0; v < VEC; ++v) {
+                    float col[U][1];
+#pragma unroll
+                    for (int u = 0; u < U; ++u) col[u][0] = e[u][v];
+                    run[v].batch(col, U, (int32_t)(k - k0), kWarps, 0);
+                }
+            } else {
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+#pragma unroll
+                    for (int v = 0; v < VEC; ++v) {
+                        if constexpr (is_var(OP)) {  // (VEC == 1: both halves the same)
+                            if (v % 2 == 0) var[v / 2].take2(VarAcc::pack(e[u][v], e[u][v + (VEC > 1)]));
+                        } else if constexpr (OP == PROD) {
+                            prod[v] *= (double)e[u][v];
+                        } else {
+                            sum_elem_c<OP>(acc[v], e[u][v], m[v], md[v]);
+                        }
+                    }
             }
-        }
+        };
+        auto sweep = [&]() {
+            int64_t k = k0 + wid;
+            for (; k + (kRows - 1) * kWarps < k1; k += kRows * kWarps) {
+                float e[kRows][VEC];
+#pragma unroll
+                for (int u = 0; u < kRows; ++u) load(k + u * kWarps, e[u]);
+                take(e, k);
+            }
+            for (; k < k1; k += kWarps) {
+                float e[1][VEC];
+                load(k, e[0]);
+                take(e, k);
+            }
+        };
 #pragma unroll
         for (int v = 0; v < VEC; ++v) {
-            const int64_t o = l + v + lo * h;
-            Partial r;
-            if (is_sum(OP)) r.d = (double)acc[v].s + (double)acc[v].c;
-            else if (OP == PROD) r.d = prod[v];
-            else r.b = run[v].to_best(k0);
-            if (FINAL) {
-                if (is_sum(OP)) fold_put<OP>(out, out64, o, lo * hi, r.d, inner, cen);
-                else if (OP == PROD) { out[o] = (float)r.d; if (out64) out64[o] = r.d; }
-                else { out[o] = r.b.v; if (index) index[o] = r.b.ifirst; }
-            } else {
-                part[o * q + c] = r;
+            acc[v] = CSum{0.0f, 0.0f};
+            prod[v] = 1.0;
+            m[v] = OP == MEANAD && live ? cen[l + v + lo * h] : 0.0f;
+            md[v] = OP == MEANAD && live ? cen[lo * hi + l + v + lo * h] : 0.0f;
+        }
+        if constexpr (is_var(OP)) {
+            if (live) load(k0, piv);
+            start();
+        }
+        if (live) sweep();
+        // warps combine: thread i finishes output i of the block's
+        __shared__ Partial s_part[kWarps][32 * VEC];
+        auto give = [&]() {
+#pragma unroll
+            for (int v = 0; v < VEC; ++v) {
+                Partial &r = s_part[wid][lane * VEC + v];
+                if constexpr (is_var(OP)) {
+                    const VarAcc &a = var[v / 2];
+                    r.v = Sums{CSum{VarAcc::half(a.s1, v & 1), VarAcc::half(a.c1, v & 1)},
+                               CSum{VarAcc::half(a.s2, v & 1), VarAcc::half(a.c2, v & 1)}, piv[v]};
+                } else if constexpr (EXT) {
+                    r.b = run[v].to_best(k0);
+                } else if constexpr (OP == PROD) {
+                    r.d = prod[v];
+                } else {
+                    r.v.s1 = acc[v];
+                }
+            }
+            __syncthreads();
+        };
+        auto together = [&](int i) {
+            Partial r = s_part[0][i];
+#pragma unroll
+            for (int w = 1; w < kWarps; ++w) {
+                const Partial &o = s_part[w][i];
+                if constexpr (is_sum(OP)) csum_merge(r.v.s1, o.v.s1);
+                if constexpr (is_var(OP)) csum_merge(r.v.s2, o.v.s2);
+                if constexpr (OP == PROD) r.d *= o.d;
+                if constexpr (EXT) r.b = best_merge<MX>(r.b, o.b);
+            }
+            return r;
+        };
+        give();
+        const int i = threadIdx.x;
+        Partial r;
+        if (i < 32 * VEC) r = together(i);
+        if constexpr (is_var(OP)) {
+            __shared__ float s_mean[32 * VEC];
+            const bool over = i < 32 * VEC && VarAcc::over(r.v);
+            if (i < 32 * VEC) s_mean[i] = over ? VarAcc::mean(r.v, k1 - k0) : r.v.piv;
+            if (__syncthreads_or(over)) {
+#pragma unroll
+                for (int v = 0; v < VEC; ++v) piv[v] = s_mean[lane * VEC + v];
+                start();
+                if (live) sweep();
+                give();
+                if (i < 32 * VEC) r = together(i);
             }
         }
+        const int64_t ti = t0 + i / VEC;
+        if (i < 32 * VEC && ti < lv * hi) {
+            const int64_t hh = ti / lv, o = (ti - hh * lv) * VEC + i % VEC + lo * hh;
+            if (FINAL) {
+                Total<OP> t;
+                t.add(r, (double)inner);
+                t.put(out, index, out64, o, lo * hi, inner, cen);
+            } else {
+                part[c * (lo * hi) + o] = r;
+            }
+        }
+        __syncthreads();
     }
 }
 

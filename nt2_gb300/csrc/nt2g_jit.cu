@@ -382,7 +382,7 @@ std::string jit_source(const std::vector<nt2g_op> &ops, const std::vector<uint8_
 // bodies of nt2g_fold_kernels.cuh are instantiated over it for op.  The NT2
 // policy folds in index order (fold_nt2) only; the fast policy and NT2's
 // elements under the compensated fold also get the short-segment, contiguous
-// (FINAL x IDX) and strided (VEC x FINAL) kernels.
+// (threads a segment x IDX) and strided (VEC x FINAL) kernels.
 std::string jit_fold_source(const std::vector<nt2g_op> &ops, const std::vector<uint8_t> &logical, int precision,
                             int op)
 {
@@ -397,8 +397,11 @@ std::string jit_fold_source(const std::vector<nt2g_op> &ops, const std::vector<u
     emit_body(s, ops, logical);
     s += "}\n\n";
     s += precision == NT2G_PREC_FAST ? "typedef nt2g::Fast P;\n" : "typedef nt2g::Nt2 P;\n";
-    s += "struct ExprSrc {\n"
-         "    JitArgs a;\n"
+    // vectors a thread has in flight: about four loads, the tables counted
+    int tables = 0;
+    for (const nt2g_op &o : ops) tables += o.code == NT2G_OP_LOAD;
+    s += "struct ExprSrc {\n    static constexpr int kBatch = " + std::string(tables <= 1 ? "4" : "2") +
+         ";\n    JitArgs a;\n"
          "    __device__ __forceinline__ float at(long long pos) const { float o[4]; jit_value<P, false, 1>(a, pos, 1, o); "
          "return o[0]; }\n"
          "    __device__ __forceinline__ float4 at4(long long pos) const { float o[4]; jit_value<P, true, 4>(a, pos, 4, o); "
@@ -413,16 +416,17 @@ std::string jit_fold_source(const std::vector<nt2g_op> &ops, const std::vector<u
     s += "extern \"C\" __global__ void __launch_bounds__(256) fold_short(const JitArgs a, long long inner, long long hi, "
          "float *out, long long *index, const float *cen, double *out64)\n"
          "{ nt2g::fold::short_body<ExprSrc, NT2G_FOP>(ExprSrc{a}, inner, hi, out, index, cen, out64); }\n";
-    for (int fin = 0; fin < 2; ++fin)
-        for (int idx = 0; idx < 2; ++idx) {
-            const std::string F = fin ? "true" : "false", I = idx ? "true" : "false";
-            s += "extern \"C\" __global__ void __launch_bounds__(256) fold_inner_" + std::to_string(fin) +
-                 std::to_string(idx) +
+    // threads a segment by whether a segment is one chunk; max and min with positions too ("x")
+    static const struct { const char *name, *final, *group; } inner[4] = {
+        {"01", "true", "8"}, {"11", "true", "32"}, {"21", "true", "256"}, {"20", "false", "256"}};
+    const bool extreme = op == NT2G_FOLD_MAX || op == NT2G_FOLD_MIN;
+    for (const auto &k : inner)
+        for (int idx = 0; idx < (extreme ? 2 : 1); ++idx)
+            s += std::string("extern \"C\" __global__ void __launch_bounds__(256) fold_inner_") + k.name + (idx ? "x" : "") +
                  "(const JitArgs a, long long inner, long long hi, long long chunk, long long q, int vec, Partial *part, "
                  "float *out, long long *index, const float *cen, double *out64)\n"
-                 "{ nt2g::fold::inner_body<ExprSrc, NT2G_FOP, " + F + ", " + I +
-                 ">(ExprSrc{a}, inner, hi, chunk, q, vec, part, out, index, cen, out64); }\n";
-        }
+                 "{ nt2g::fold::inner_body<ExprSrc, NT2G_FOP, " + k.final + ", " + (idx ? "true" : "false") + ", " +
+                 k.group + ">(ExprSrc{a}, inner, hi, chunk, q, vec, part, out, index, cen, out64); }\n";
     for (int v4 = 0; v4 < 2; ++v4)
         for (int fin = 0; fin < 2; ++fin) {
             const std::string V = v4 ? "4" : "1", F = fin ? "true" : "false";
@@ -945,12 +949,18 @@ const JitFoldKernels *jit_fold_kernels(const std::vector<nt2g_op> &ops, const st
             if (ce == cudaSuccess) ce = cudaLibraryGetKernel(&e.k.nt2, e.lib, "fold_nt2");
             if (precision != NT2G_PREC_NT2) {
                 if (ce == cudaSuccess) ce = cudaLibraryGetKernel(&e.k.shrt, e.lib, "fold_short");
+                static const char *const inner[4] = {"01", "11", "21", "20"};
+                const bool extreme = op == NT2G_FOLD_MAX || op == NT2G_FOLD_MIN;
+                for (int a = 0; a < 4; ++a)
+                    for (int b = 0; b < (extreme ? 2 : 1); ++b)
+                        if (ce == cudaSuccess)
+                            ce = cudaLibraryGetKernel(&e.k.inner[a][b], e.lib,
+                                                      (std::string("fold_inner_") + inner[a] + (b ? "x" : "")).c_str());
                 for (int a = 0; a < 2; ++a)
-                    for (int b = 0; b < 2; ++b) {
-                        const std::string ab = std::to_string(a) + std::to_string(b);
-                        if (ce == cudaSuccess) ce = cudaLibraryGetKernel(&e.k.inner[a][b], e.lib, ("fold_inner_" + ab).c_str());
-                        if (ce == cudaSuccess) ce = cudaLibraryGetKernel(&e.k.outer[a][b], e.lib, ("fold_outer_" + ab).c_str());
-                    }
+                    for (int b = 0; b < 2; ++b)
+                        if (ce == cudaSuccess)
+                            ce = cudaLibraryGetKernel(&e.k.outer[a][b], e.lib,
+                                                      ("fold_outer_" + std::to_string(a) + std::to_string(b)).c_str());
             }
             if (ce == cudaSuccess) {
                 e.ok = true;
