@@ -55,7 +55,7 @@ class Node:
 # var > d, which computes the same but no longer has the expression's shape.
 def Table(tensor):
     """A device table leaf (CUDA tensor, float32 or uint8)."""
-    import torch
+    torch = lib._pytorch()
     if tensor.dtype not in (torch.uint8, torch.float32):
         raise TypeError(f"tables hold float32 or uint8, not {tensor.dtype}")
     return Node("LOAD", (), lib.U8 if tensor.dtype == torch.uint8 else lib.F32, table=tensor)
@@ -691,29 +691,34 @@ def lower(outs, exprs, fold=None):
         return slot_of[key]
 
     ops, memo = [], {}
+    code = lib.OP
 
     def emit(n):
+        op = n.op
         # table loads are never memoised here: a load after a store to the
         # same table must see the stored value (tie semantics); the library's
         # compiler forwards and deduplicates them
-        if n.op != "LOAD" and id(n) in memo:
-            return memo[id(n)]
-        if n.op == "LOAD":
-            s = slot(("t", n.table.data_ptr(), n.table.dtype), n.table)
-            ops.append((lib.OP["LOAD"], n.dtype, s, -1, -1, 0.0))
-        elif n.op == "SCALAR":
-            s = slot(("s", id(n)), n)
-            ops.append((lib.OP["SCALAR"], n.dtype, s, -1, -1, 0.0))
-        elif n.op == "CONST":
-            ops.append((lib.OP["CONST"], n.dtype, -1, -1, -1, n.imm))
-        elif n.op == "INDEX":
-            ops.append((lib.OP["INDEX"], n.dtype, -1, -1, -1, 0.0))
+        if op == "LOAD":
+            t = n.table
+            ops.append((code["LOAD"], n.dtype, slot(("t", t.data_ptr(), t.dtype), t), -1, -1, 0.0))
+            return len(ops) - 1
+        k = memo.get(id(n))
+        if k is not None:
+            return k
+        if op == "SCALAR":
+            ops.append((code["SCALAR"], n.dtype, slot(("s", id(n)), n), -1, -1, 0.0))
+        elif op == "CONST":
+            ops.append((code["CONST"], n.dtype, -1, -1, -1, n.imm))
+        elif op == "INDEX":
+            ops.append((code["INDEX"], n.dtype, -1, -1, -1, 0.0))
         else:
-            a = [emit(x) for x in n.args] + [-1, -1, -1]
-            dt = _compare_dtype(n) if n.op in _LOGICAL_OPS else n.dtype
-            ops.append((lib.OP[n.op], dt, a[0], a[1], a[2], 0.0))
-        memo[id(n)] = len(ops) - 1
-        return memo[id(n)]
+            args = n.args
+            a = emit(args[0])
+            b = emit(args[1]) if len(args) > 1 else -1
+            c = emit(args[2]) if len(args) > 2 else -1
+            ops.append((code[op], _compare_dtype(n) if op in _LOGICAL_OPS else n.dtype, a, b, c, 0.0))
+        memo[id(n)] = k = len(ops) - 1
+        return k
 
     for o, e in zip(outs, exprs):
         v = emit(e)
@@ -791,17 +796,9 @@ def assign(outs, exprs, precision=lib.PREC_FAST, offset=0, count=None, force_gen
     force_generic: False/0 = bound fused kernel, else the run-time compiled
     kernel, else the interpreter; True/1 = compiled kernel, else interpreter;
     2 = interpreter only."""
-    import torch
     outs, exprs = list(outs), list(exprs)
     prog, slots = compile_program(outs, exprs)
-    args = (lib.Arg * len(slots))()
-    n = None
-    for i, s in enumerate(slots):
-        if isinstance(s, Node):  # a SCALAR leaf
-            args[i] = lib.Arg(None, s.imm, s.dtype, 1)
-        else:
-            n = s.numel() if n is None else min(n, s.numel())
-            args[i] = lib.Arg(s.data_ptr(), 0.0, lib.U8 if s.dtype == torch.uint8 else lib.F32, 0)
+    args, n = _args_of(slots)
     if count is None:
         count = n - offset
         _check_generative_sizes(exprs, count)
@@ -811,7 +808,7 @@ def assign(outs, exprs, precision=lib.PREC_FAST, offset=0, count=None, force_gen
 
 
 def _args_of(slots):
-    import torch
+    torch = lib._pytorch()
     args = (lib.Arg * len(slots))()
     n = None
     for i, s in enumerate(slots):
@@ -824,13 +821,15 @@ def _args_of(slots):
 
 
 def _slot_of(slots, x):
-    import torch
-    for i, s in enumerate(slots):
-        if isinstance(x, torch.Tensor):
-            if not isinstance(s, Node) and s.data_ptr() == x.data_ptr() and s.dtype == x.dtype:
+    if isinstance(x, Node):
+        for i, s in enumerate(slots):
+            if s is x:
                 return i
-        elif s is x:
-            return i
+    else:
+        at, dtype = x.data_ptr(), x.dtype
+        for i, s in enumerate(slots):
+            if not isinstance(s, Node) and s.data_ptr() == at and s.dtype == dtype:
+                return i
     raise ValueError("not an argument of the program")
 
 
