@@ -39,8 +39,15 @@ constexpr int64_t kSmallSeg = 64;        // (many) segments up to this length: o
 struct RawSrc {
     static constexpr int kBatch = 4;  // vectors a thread has in flight
     const float *x;
+    typedef float4 Raw;
     __device__ __forceinline__ float at(int64_t pos) const { return ld_stream(x + pos); }
-    __device__ __forceinline__ float4 at4(int64_t pos) const { return ld_stream((const float4 *)(x + pos)); }
+    __device__ __forceinline__ Raw fetch(int64_t pos) const { return make_float4(ld_stream(x + pos), 0.0f, 0.0f, 0.0f); }
+    __device__ __forceinline__ Raw fetch4(int64_t pos) const { return ld_stream((const float4 *)(x + pos)); }
+    __device__ __forceinline__ float value(const Raw &r, int64_t) const { return r.x; }
+    __device__ __forceinline__ void value4(const Raw &r, int64_t, float (&e)[4]) const
+    {
+        e[0] = r.x; e[1] = r.y; e[2] = r.z; e[3] = r.w;
+    }
 };
 
 template <int OP, bool FINAL, bool IDX, int G>

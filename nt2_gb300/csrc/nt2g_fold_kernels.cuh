@@ -4,9 +4,12 @@
 // (column-major), folding over `inner`: out[l + lo*h] = fold_k x(l + lo*(k + inner*h)).
 //
 // The element values come from a source type Src with
-//   float  at(int64_t pos)   the element at linear position pos
-//   float4 at4(int64_t pos)  the four elements pos .. pos+3 (pos a multiple of 4;
-//                            only called when the source is 16-byte addressable)
+//   float at(int64_t pos)      the element at linear position pos
+//   Raw fetch(int64_t pos)     what it is made of, loaded; fetch4: of the four
+//                              elements pos .. pos+3 (pos a multiple of 4; only
+//                              called when the source is 16-byte addressable)
+//   float value(Raw, pos), value4(Raw, pos, float (&)[4])  the elements
+//   kBatch                     fetches a thread has in flight
 // The library instantiates the bodies over a table (nt2g_fold.cu); the
 // run-time compiler instantiates them over a compiled expression, so a fold of
 // an expression (sum(exp(x)*y), sum(abs(x - y), 1), ...) evaluates every
@@ -590,12 +593,17 @@ __device__ __forceinline__ void inner_body(const Src &src, int64_t inner, int64_
                 for (int64_t j = a; j < b; j += kBatch * G) {
                     const int64_t left = b - j - tid;
                     float e[kBatch][4];
+                    typename Src::Raw raw[kBatch];
                     const int n = left <= 0 ? 0 : left > (kBatch - 1) * G ? kBatch : (int)((left + G - 1) / G);
 #pragma unroll
                     for (int u = 0; u < kBatch; ++u) {  // (past the end: the last one again, so that no load waits for a branch)
                         const int64_t at = j + tid + u * G;
-                        const float4 f = src.at4(4 * (at < b ? at : b - 1));
-                        e[u][0] = f.x; e[u][1] = f.y; e[u][2] = f.z; e[u][3] = f.w;
+                        raw[u] = src.fetch4(4 * (at < b ? at : b - 1));
+                    }
+#pragma unroll
+                    for (int u = 0; u < kBatch; ++u) {
+                        const int64_t at = j + tid + u * G;
+                        src.value4(raw[u], 4 * (at < b ? at : b - 1), e[u]);
                     }
                     const int32_t pos = (int32_t)(4 * (j + tid) - p0);
                     if (j + kBatch * G <= b) take(e, kBatch, pos, 4 * G);
@@ -614,11 +622,17 @@ __device__ __forceinline__ void inner_body(const Src &src, int64_t inner, int64_
                 for (int64_t j = p0; j < p1; j += kBatch * G) {
                     const int64_t left = p1 - j - tid;
                     float e[kBatch][1];
+                    typename Src::Raw raw[kBatch];
                     const int n = left <= 0 ? 0 : left > (kBatch - 1) * G ? kBatch : (int)((left + G - 1) / G);
 #pragma unroll
                     for (int u = 0; u < kBatch; ++u) {
                         const int64_t at = j + tid + u * G;
-                        e[u][0] = src.at(at < p1 ? at : p1 - 1);
+                        raw[u] = src.fetch(at < p1 ? at : p1 - 1);
+                    }
+#pragma unroll
+                    for (int u = 0; u < kBatch; ++u) {
+                        const int64_t at = j + tid + u * G;
+                        e[u][0] = src.value(raw[u], at < p1 ? at : p1 - 1);
                     }
                     take(e, n, (int32_t)(j + tid - p0), G);
                 }
@@ -767,13 +781,13 @@ __device__ __forceinline__ void outer_body(const Src &src, int64_t lo, int64_t i
 #pragma unroll
             for (int v = 0; v < VEC; v += 2) var[v / 2].start(piv[v], piv[v + (VEC > 1)]);
         };
-        auto load = [&](int64_t k, float (&e)[VEC]) {
-            if constexpr (VEC == 4) {
-                const float4 f = src.at4(base + lo * k);
-                e[0] = f.x; e[1] = f.y; e[2] = f.z; e[3] = f.w;
-            } else {
-                e[0] = src.at(base + lo * k);
-            }
+        auto fetch = [&](int64_t k) {
+            if constexpr (VEC == 4) return src.fetch4(base + lo * k);
+            else return src.fetch(base + lo * k);
+        };
+        auto value = [&](const typename Src::Raw &r, int64_t k, float (&e)[VEC]) {
+            if constexpr (VEC == 4) src.value4(r, base + lo * k, e);
+            else e[0] = src.value(r, base + lo * k);
         };
         // rows k, k + kWarps, ...
         auto take = [&](const auto &e, int64_t k) {
@@ -805,13 +819,16 @@ __device__ __forceinline__ void outer_body(const Src &src, int64_t lo, int64_t i
             int64_t k = k0 + wid;
             for (; k + (kRows - 1) * kWarps < k1; k += kRows * kWarps) {
                 float e[kRows][VEC];
+                typename Src::Raw raw[kRows];
 #pragma unroll
-                for (int u = 0; u < kRows; ++u) load(k + u * kWarps, e[u]);
+                for (int u = 0; u < kRows; ++u) raw[u] = fetch(k + u * kWarps);
+#pragma unroll
+                for (int u = 0; u < kRows; ++u) value(raw[u], k + u * kWarps, e[u]);
                 take(e, k);
             }
             for (; k < k1; k += kWarps) {
                 float e[1][VEC];
-                load(k, e[0]);
+                value(fetch(k), k, e[0]);
                 take(e, k);
             }
         };
@@ -823,7 +840,7 @@ __device__ __forceinline__ void outer_body(const Src &src, int64_t lo, int64_t i
             md[v] = OP == MEANAD && live ? cen[lo * hi + l + v + lo * h] : 0.0f;
         }
         if constexpr (is_var(OP)) {
-            if (live) load(k0, piv);
+            if (live) value(fetch(k0), k0, piv);
             start();
         }
         if (live) sweep();

@@ -31,6 +31,8 @@
 #include "nt2g_accum_src.h"  // kNt2gAccumSrc: nt2g_accum.cuh
 #include "nt2g_fold_src.h"   // kNt2gFoldSrc: nt2g_fold_kernels.cuh
 #include "nt2g_vjp_src.h"    // kNt2gVjpSrc: nt2g_vjp.cuh
+#include "nt2g_f2_src.h"     // kNt2gF2Src: nt2g_f2.cuh
+#include "nt2g_lanes_src.h"  // kNt2gLanesSrc: nt2g_lanes.cuh
 
 namespace nt2g {
 
@@ -88,11 +90,30 @@ static const char kJitPrelude[] = R"NT2G_SRC(
 struct JitArgs { void *ptr[16]; float scal[16]; unsigned scal_u8[16]; int dtype[16]; long long pos0; };
 #define NT2G_L _Pragma("unroll") for (int j = 0; j < 4; ++j)
 #define NT2G_LL _Pragma("unroll") for (int j = 0; j < L; ++j)
+#define NT2G_V(x) nt2g::lane::Of<L, A>{x}
 template <bool FULL> __device__ __forceinline__ void jit_ldf(float (&d)[4], const void *p, long long i, int cnt)
 {
     const float *q = (const float *)p + i;
     if (FULL) { float4 t = __ldcs((const float4 *)q); d[0] = t.x; d[1] = t.y; d[2] = t.z; d[3] = t.w; }
     else { NT2G_L d[j] = j < cnt ? q[j] : 0.0f; }
+}
+template <bool FULL> __device__ __forceinline__ void jit_ldf(float (&d)[2], const void *p, long long i, int cnt)
+{
+    const float *q = (const float *)p + i;
+    if (FULL) { const float2 t = __ldcs((const float2 *)q); d[0] = t.x; d[1] = t.y; }
+    else { d[0] = q[0]; d[1] = cnt > 1 ? q[1] : 0.0f; }
+}
+template <bool FULL> __device__ __forceinline__ void jit_stf(void *p, long long i, int cnt, const float (&v)[2])
+{
+    float *q = (float *)p + i;
+    if (FULL) __stcs((float2 *)q, make_float2(v[0], v[1]));
+    else { q[0] = v[0]; if (cnt > 1) q[1] = v[1]; }
+}
+template <bool FULL> __device__ __forceinline__ void jit_ldb(unsigned (&d)[2], const void *p, long long i, int cnt)
+{
+    const unsigned char *q = (const unsigned char *)p + i;
+    if (FULL) { const unsigned w = *(const unsigned short *)q; d[0] = w & 255u; d[1] = w >> 8; }
+    else { d[0] = q[0]; d[1] = cnt > 1 ? q[1] : 0u; }
 }
 template <bool FULL> __device__ __forceinline__ void jit_ldb(unsigned (&d)[4], const void *p, long long i, int cnt)
 {
@@ -155,11 +176,29 @@ static std::string fconst(float f)
     return b;
 }
 
+// The function of nt2g_lanes.cuh that evaluates an opcode over all lanes of a
+// thread (nullptr: one lane at a time, by nt2g_math.cuh).
+static const char *lane_function(int code)
+{
+    switch (code) {
+    case NT2G_OP_EXP: return "exp";
+    case NT2G_OP_LOG: return "log";
+    case NT2G_OP_SIN: return "sin";
+    case NT2G_OP_COS: return "cos";
+    case NT2G_OP_POW: return "pow";
+    case NT2G_OP_ERF: return "erf";
+    case NT2G_OP_GAMMALN: return "gammaln";
+    case NT2G_OP_NORMCDF: return "normcdf";
+    case NT2G_OP_FASTNORMCDF: return "fastnormcdf";
+    default: return nullptr;
+    }
+}
+
 // The statements of a program over L lanes (4 consecutive elements per call
 // in a transform; 1 or 4 in a fold's element function).  STORE writes the
 // output tables; FOLD (fold programs) hands the folded value to out[].
 static void emit_body(std::string &s, const std::vector<nt2g_op> &ops, const std::vector<uint8_t> &logical,
-                      bool stores = true)
+                      bool stores = true, bool fetched = false)
 {
     auto v = [](int x) { return "v" + std::to_string(x) + "[j]"; };
     // every table load first, so a tile's memory requests are in flight while its
@@ -169,6 +208,11 @@ static void emit_body(std::string &s, const std::vector<nt2g_op> &ops, const std
         const nt2g_op &o = ops[k];
         if (o.code != NT2G_OP_LOAD) continue;
         const bool f32 = o.dtype == NT2G_F32;
+        if (fetched) {  // a fold's loads, issued by jit_fetch
+            const std::string v = "v" + std::to_string(k);
+            s += std::string(f32 ? "    const float (&" : "    const unsigned (&") + v + ")[A] = in." + v + ";\n";
+            continue;
+        }
         s += (f32 ? "    float v" : "    unsigned v") + std::to_string(k) + "[A]; " +
              (f32 ? "jit_ldf<FULL>(v" : "jit_ldb<FULL>(v") + std::to_string(k) + ", a.ptr[" + std::to_string(o.a) +
              "], i, cnt);\n";
@@ -203,12 +247,26 @@ static void emit_body(std::string &s, const std::vector<nt2g_op> &ops, const std
             // the positive side is the one whose argument is y itself
             const bool k_is_neg = ops[o.a].code == NT2G_OP_NEG && ops[o.a].a == ops[p].a;
             const int pos = k_is_neg ? p : (int)k, neg = k_is_neg ? (int)k : p;
-            s += "    float v" + std::to_string(k) + "[A], v" + std::to_string(p) + "[A]; NT2G_LL nt2g::normcdf_pair<P>(" +
-                 v(ops[pos].a) + ", " + v(pos) + ", " + v(neg) + ");\n";
+            const std::string at = std::to_string(ops[pos].a);
+            s += "    float v" + std::to_string(k) + "[A], v" + std::to_string(p) + "[A]; ";
+            if (logical[ops[pos].a] || ops[ops[pos].a].dtype != NT2G_F32)
+                s += "NT2G_LL nt2g::normcdf_pair<P>(" + v(ops[pos].a) + ", " + v(pos) + ", " + v(neg) + ");\n";
+            else
+                s += "nt2g::normcdf_pair<P>(NT2G_V(v" + at + "), NT2G_V(v" + std::to_string(pos) + "), NT2G_V(v" +
+                     std::to_string(neg) + "));\n";
             continue;
         }
         const std::string A = o.a >= 0 ? v(o.a) : "", B = o.b >= 0 ? v(o.b) : "", C = o.c >= 0 ? v(o.c) : "";
         const std::string slot = std::to_string(o.a);
+        if (const char *fn = lane_function(o.code)) {  // all lanes at once
+            const bool two = o.code == NT2G_OP_POW;
+            auto floats = [&](int x) { return !logical[x] && ops[x].dtype == NT2G_F32; };
+            if (floats(o.a) && (!two || floats(o.b))) {
+                s += "    float v" + std::to_string(k) + "[A]; nt2g::lane::" + fn + "<P, L>(v" + slot +
+                     (two ? ", v" + std::to_string(o.b) : "") + ", v" + std::to_string(k) + ");\n";
+                continue;
+            }
+        }
         std::string e;
         switch (o.code) {
         case NT2G_OP_LOAD: continue;  // emitted above
@@ -361,6 +419,8 @@ std::string jit_source(const std::vector<nt2g_op> &ops, const std::vector<uint8_
     std::string s;
     s.reserve(sizeof kJitPrelude + 40000 + ops.size() * 96);
     s += kNt2gMathSrc;
+    s += kNt2gF2Src;
+    s += kNt2gLanesSrc;
     s += kJitPrelude;
     s += "template <class P, bool FULL>\n__device__ __forceinline__ void jit_tile(const JitArgs &a, long long i, int cnt)\n{\n"
          "    constexpr int L = 4, A = 4;\n";
@@ -389,12 +449,28 @@ std::string jit_fold_source(const std::vector<nt2g_op> &ops, const std::vector<u
     std::string s;
     s.reserve(sizeof kJitPrelude + sizeof kNt2gAccumSrc + sizeof kNt2gFoldSrc + 40000 + ops.size() * 96);
     s += kNt2gMathSrc;
+    s += kNt2gF2Src;
+    s += kNt2gLanesSrc;
     s += kJitPrelude;
     s += kNt2gAccumSrc;
     s += kNt2gFoldSrc;
-    s += "template <class P, bool FULL, int L>\n__device__ __forceinline__ void jit_value(const JitArgs &a, long long i, "
-         "int cnt, float (&out)[4])\n{\n    constexpr int A = 4;\n";
-    emit_body(s, ops, logical);
+    // an element's table values and what is made of them, apart: a thread has
+    // all its loads in flight before the first value, whose special cases branch
+    s += "struct JitIn {\n";
+    std::string fetch;
+    for (size_t k = 0; k < ops.size(); ++k) {
+        if (ops[k].code != NT2G_OP_LOAD) continue;
+        const bool f32 = ops[k].dtype == NT2G_F32;
+        const std::string v = "v" + std::to_string(k);
+        s += (f32 ? "    float " : "    unsigned ") + v + "[4];\n";
+        fetch += std::string(f32 ? "    jit_ldf<FULL>(in." : "    jit_ldb<FULL>(in.") + v + ", a.ptr[" +
+                 std::to_string(ops[k].a) + "], i, cnt);\n";
+    }
+    s += "};\ntemplate <bool FULL>\n__device__ __forceinline__ void jit_fetch(const JitArgs &a, long long i, int cnt, JitIn &in)\n{\n" +
+         fetch + "}\n";
+    s += "template <class P, int L>\n__device__ __forceinline__ void jit_value(const JitArgs &a, const JitIn &in, long long i, "
+         "float (&out)[4])\n{\n    constexpr int A = 4;\n";
+    emit_body(s, ops, logical, true, true);
     s += "}\n\n";
     s += precision == NT2G_PREC_FAST ? "typedef nt2g::Fast P;\n" : "typedef nt2g::Nt2 P;\n";
     // vectors a thread has in flight: about four loads, the tables counted
@@ -402,10 +478,14 @@ std::string jit_fold_source(const std::vector<nt2g_op> &ops, const std::vector<u
     for (const nt2g_op &o : ops) tables += o.code == NT2G_OP_LOAD;
     s += "struct ExprSrc {\n    static constexpr int kBatch = " + std::string(tables <= 1 ? "4" : "2") +
          ";\n    JitArgs a;\n"
-         "    __device__ __forceinline__ float at(long long pos) const { float o[4]; jit_value<P, false, 1>(a, pos, 1, o); "
+         "    typedef JitIn Raw;\n"
+         "    __device__ __forceinline__ Raw fetch(long long pos) const { Raw r; jit_fetch<false>(a, pos, 1, r); return r; }\n"
+         "    __device__ __forceinline__ Raw fetch4(long long pos) const { Raw r; jit_fetch<true>(a, pos, 4, r); return r; }\n"
+         "    __device__ __forceinline__ float value(const Raw &r, long long pos) const { float o[4]; jit_value<P, 1>(a, r, pos, o); "
          "return o[0]; }\n"
-         "    __device__ __forceinline__ float4 at4(long long pos) const { float o[4]; jit_value<P, true, 4>(a, pos, 4, o); "
-         "return make_float4(o[0], o[1], o[2], o[3]); }\n"
+         "    __device__ __forceinline__ void value4(const Raw &r, long long pos, float (&o)[4]) const { jit_value<P, 4>(a, r, pos, "
+         "o); }\n"
+         "    __device__ __forceinline__ float at(long long pos) const { return value(fetch(pos), pos); }\n"
          "};\n";
     s += "#define NT2G_FOP " + std::to_string(op) + "\n";
     s += "using nt2g::fold::Partial;\n"
@@ -453,6 +533,8 @@ std::string jit_batch_source(const std::vector<ProgramCode> &progs, int precisio
     std::string s;
     s.reserve(sizeof kJitPrelude + 40000 + progs.size() * 4096);
     s += kNt2gMathSrc;
+    s += kNt2gF2Src;
+    s += kNt2gLanesSrc;
     s += kJitPrelude;
     s += "struct BItem { JitArgs a; long long n; int prog; int vec; };\n";
     for (size_t k = 0; k < progs.size(); ++k) {
@@ -565,8 +647,8 @@ static bool adjoint_rule(std::string &s, const std::vector<nt2g_op> &ops, int k,
         const std::string phi = "phi" + std::to_string(base);
         if (act(o.a) && !phi_done[base]) {
             phi_done[base] = 1;
-            s += "    float " + phi + "[4]; NT2G_L " + phi + "[j] = nt2g::vjp::kInvSqrt2Pi * nt2g::exp<D>(-0.5f * " +
-                 v(base) + " * " + v(base) + ");\n";
+            s += "    float " + phi + "[A]; { float t[A]; NT2G_LL t[j] = -0.5f * " + v(base) + " * " + v(base) +
+                 "; nt2g::lane::exp<D, L>(t, " + phi + "); } NT2G_LL " + phi + "[j] *= nt2g::vjp::kInvSqrt2Pi;\n";
         }
         to(o.a, G + " * " + phi + "[j]");
         break;
@@ -692,9 +774,9 @@ static bool adjoint_rule(std::string &s, const std::vector<nt2g_op> &ops, int k,
     }
     if (add.empty()) return true;
     if (pre.empty()) {
-        for (const auto &t : add) s += "    NT2G_L g" + std::to_string(t.first) + "[j] += " + t.second + ";\n";
+        for (const auto &t : add) s += "    NT2G_LL g" + std::to_string(t.first) + "[j] += " + t.second + ";\n";
     } else {
-        s += "    NT2G_L { " + pre;
+        s += "    NT2G_LL { " + pre;
         for (const auto &t : add) s += " g" + std::to_string(t.first) + "[j] += " + t.second + ";";
         s += " }\n";
     }
@@ -761,15 +843,18 @@ std::string jit_vjp_source(const std::vector<nt2g_op> &ops, const std::vector<ui
     std::string s;
     s.reserve(sizeof kJitPrelude + sizeof kNt2gVjpSrc + 40000 + ops.size() * 256);
     s += kNt2gMathSrc;
+    s += kNt2gF2Src;
+    s += kNt2gLanesSrc;
+    s += kNt2gAccumSrc;
     s += kNt2gVjpSrc;
     s += kJitPrelude;
     s += "struct VjpArgs { const float *ct[16]; float *grad[16]; };\n";
     s += "#define NT2G_NS " + std::to_string(ns > 0 ? ns : 1) + "\n";
     s += "template <class P, bool FULL>\n__device__ __forceinline__ void vjp_tile(const JitArgs &a, const VjpArgs &g, "
-         "long long i, int cnt, double (&sacc)[NT2G_NS])\n{\n    typedef nt2g::Fast D;\n    constexpr int L = 4, A = 4;\n";
+         "long long i, int cnt, nt2g::CSum (&sacc)[NT2G_NS])\n{\n    typedef nt2g::Fast D;\n    constexpr int L = 2, A = 2;\n";
     emit_body(s, ops, logical, false);
     for (size_t k = 0; k < ops.size(); ++k)
-        if (act[k]) s += "    float g" + std::to_string(k) + "[4] = {0.0f, 0.0f, 0.0f, 0.0f};\n";
+        if (act[k]) s += "    float g" + std::to_string(k) + "[A] = {0.0f, 0.0f};\n";
     // seeds: the cotangent of each output slot flows into the last value stored there
     std::vector<int> last_store(kMaxSlots, -1);
     for (size_t k = 0; k < ops.size(); ++k)
@@ -778,7 +863,7 @@ std::string jit_vjp_source(const std::vector<nt2g_op> &ops, const std::vector<ui
         const int st = last_store[slot];
         if (st < 0 || !act[ops[st].a]) continue;
         const std::string sl = std::to_string(slot), val = std::to_string(ops[st].a);
-        s += "    if (g.ct[" + sl + "]) { float t[4]; jit_ldf<FULL>(t, g.ct[" + sl + "], i, cnt); NT2G_L g" + val +
+        s += "    if (g.ct[" + sl + "]) { float t[A]; jit_ldf<FULL>(t, g.ct[" + sl + "], i, cnt); NT2G_LL g" + val +
              "[j] += t[j]; }\n";
     }
     std::vector<uint8_t> phi_done(ops.size(), 0);
@@ -807,29 +892,29 @@ std::string jit_vjp_source(const std::vector<nt2g_op> &ops, const std::vector<ui
         if (!read_f32[slot]) continue;
         const std::string sl = std::to_string(slot);
         const std::string val = grad_of[slot].empty() ? "0.0f" : grad_of[slot];  // no output depends on it
-        s += "    if (g.grad[" + sl + "]) { float t[4]; NT2G_L t[j] = " + val + "; jit_stf<FULL>(g.grad[" + sl +
+        s += "    if (g.grad[" + sl + "]) { float t[A]; NT2G_LL t[j] = " + val + "; jit_stf<FULL>(g.grad[" + sl +
              "], i, cnt, t); }\n";
     }
     for (int q = 0; q < ns; ++q)
         for (size_t k = 0; k < ops.size(); ++k)
             if (ops[k].code == NT2G_OP_SCALAR && act[k] && ops[k].a == sslots[q])
-                s += "    NT2G_L if (j < cnt) sacc[" + std::to_string(q) + "] += (double)g" + std::to_string(k) + "[j];\n";
+                s += "    NT2G_LL if (j < cnt) nt2g::csum_add(sacc[" + std::to_string(q) + "], g" + std::to_string(k) + "[j]);\n";
     s += "}\n\n";
     s += "extern \"C\" __global__ void __launch_bounds__(256) nt2g_vjp_kernel(const JitArgs a, const VjpArgs g, "
          "long long n, int vec, double *partials)\n{\n";
     s += precision == NT2G_PREC_NT2 ? "    typedef nt2g::Nt2 P;\n" : "    typedef nt2g::Fast P;\n";
-    s += "    double sacc[NT2G_NS];\n"
-         "    for (int q = 0; q < NT2G_NS; ++q) sacc[q] = 0.0;\n"
-         "    const long long stride = (long long)gridDim.x * blockDim.x * 4;\n"
-         "    for (long long i = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * 4; i < n; i += stride) {\n"
-         "        const int cnt = n - i < 4 ? (int)(n - i) : 4;\n"
-         "        if (vec && cnt == 4) vjp_tile<P, true>(a, g, i, 4, sacc);\n"
+    s += "    nt2g::CSum sacc[NT2G_NS];\n"
+         "    for (int q = 0; q < NT2G_NS; ++q) sacc[q] = nt2g::CSum{0.0f, 0.0f};\n"
+         "    const long long stride = (long long)gridDim.x * blockDim.x * 2;\n"
+         "    for (long long i = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * 2; i < n; i += stride) {\n"
+         "        const int cnt = n - i < 2 ? (int)(n - i) : 2;\n"
+         "        if (vec && cnt == 2) vjp_tile<P, true>(a, g, i, 2, sacc);\n"
          "        else vjp_tile<P, false>(a, g, i, cnt, sacc);\n"
          "    }\n";
     if (ns > 0)
         s += "    __shared__ double red[8][NT2G_NS];\n"
              "    for (int q = 0; q < NT2G_NS; ++q) {\n"
-             "        double x = sacc[q];\n"
+             "        double x = (double)sacc[q].s + (double)sacc[q].c;\n"
              "        for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);\n"
              "        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5][q] = x;\n"
              "    }\n"

@@ -12,76 +12,9 @@
 // MUFU approximations stay per lane.
 #pragma once
 #include "nt2g_exprs.cuh"
+#include "nt2g_lanes.cuh"
 
 namespace nt2g {
-
-struct f2 {
-    unsigned long long v;
-};
-
-__device__ __forceinline__ f2 pk(float lo, float hi)
-{
-    f2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(lo), "f"(hi));
-    return r;
-}
-__device__ __forceinline__ void upk(f2 a, float &lo, float &hi)
-{
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(a.v));
-}
-__device__ __forceinline__ f2 dup(float x) { return pk(x, x); }
-__device__ __forceinline__ f2 add2(f2 a, f2 b)
-{
-    f2 d;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d.v) : "l"(a.v), "l"(b.v));
-    return d;
-}
-__device__ __forceinline__ f2 sub2(f2 a, f2 b)
-{
-    f2 d;
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d.v) : "l"(a.v), "l"(b.v));
-    return d;
-}
-__device__ __forceinline__ f2 mul2(f2 a, f2 b)
-{
-    f2 d;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d.v) : "l"(a.v), "l"(b.v));
-    return d;
-}
-__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c)
-{
-    f2 d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d.v) : "l"(a.v), "l"(b.v), "l"(c.v));
-    return d;
-}
-// -a by flipping both sign bits (integer pipe, exact, no FP32 slot)
-__device__ __forceinline__ f2 negx2(f2 a)
-{
-    f2 r;
-    r.v = a.v ^ 0x8000000080000000ull;
-    return r;
-}
-__device__ __forceinline__ f2 neg2(f2 a) { return negx2(a); }
-template <class F> __device__ __forceinline__ f2 lanes(f2 a, F f)
-{
-    float x, y;
-    upk(a, x, y);
-    return pk(f(x), f(y));
-}
-template <class F> __device__ __forceinline__ f2 lanes(f2 a, f2 b, F f)
-{
-    float x0, x1, y0, y1;
-    upk(a, x0, x1);
-    upk(b, y0, y1);
-    return pk(f(x0, y0), f(x1, y1));
-}
-
-// Horner in NT2's coefficient order, as horner<Fast>.
-__device__ __forceinline__ f2 horner2(f2, f2 acc) { return acc; }
-template <class... R> __device__ __forceinline__ f2 horner2(f2 x, f2 acc, float c, R... rest)
-{
-    return horner2(x, fma2(x, acc, dup(c)), rest...);
-}
 
 __device__ __forceinline__ float rcp_approx(float b)
 {
@@ -112,38 +45,6 @@ __device__ __forceinline__ f2 fdiv2(f2 a, f2 b, f2 nb)
     f2 q = mul2(a, r);
     f2 e = fma2(q, nb, a);
     return fma2(e, r, q);
-}
-
-// log_pos_fast, lane for lane.
-__device__ __forceinline__ f2 log_pos_fast2(f2 z)
-{
-    float z0, z1;
-    upk(z, z0, z1);
-    const uint32_t u0 = f_bits(z0), u1 = f_bits(z1);
-    const float m0 = bits_f((u0 & 0x007fffffu) | 0x3f000000u), m1 = bits_f((u1 & 0x007fffffu) | 0x3f000000u);
-    const bool l0 = m0 < bits_f(NT2G_SQRT_2O_2), l1 = m1 < bits_f(NT2G_SQRT_2O_2);
-    f2 fe = sub2(pk(bits_f(0x4B000000u | (uint32_t)((int32_t)u0 >> 23)),
-                    bits_f(0x4B000000u | (uint32_t)((int32_t)u1 >> 23))),
-                 pk(l0 ? 8388735.0f : 8388734.0f, l1 ? 8388735.0f : 8388734.0f));
-    f2 m = pk(m0, m1);
-    f2 mm = add2(m, m);
-    float mm0, mm1;
-    upk(mm, mm0, mm1);
-    f2 x = sub2(pk(l0 ? mm0 : m0, l1 ? mm1 : m1), dup(1.0f));
-    f2 x2 = mul2(x, x);
-    f2 y = horner2(x, dup(bits_f(0xbda5dff0u)), bits_f(0x3e0229f9u), bits_f(0xbe04d6b7u), bits_f(0x3e116e80u),
-                   bits_f(0xbe2a6aa0u), bits_f(0x3e4cd0a3u), bits_f(0xbe800064u), bits_f(0x3eaaaaa9u));
-    y = mul2(mul2(y, x), x2);
-    y = fma2(fe, dup(bits_f(NT2G_LOG_2LO)), y);
-    y = fma2(dup(-0.5f), x2, y);
-    return fma2(dup(bits_f(NT2G_LOG_2HI)), fe, add2(x, y));
-}
-
-__device__ __forceinline__ f2 erfc_tail_poly2(f2 w)
-{
-    f2 d = sub2(w, dup(0.5f));
-    return horner2(d, dup(0x1.5af3d4p-5f), -0x1.38d8fcp-6f, -0x1.382c16p-4f, 0x1.c51560p-5f, 0x1.908f48p-4f,
-                   -0x1.a94032p-4f, -0x1.604ccep-3f, 0x1.2a8c2ep-3f, 0x1.1e2dc2p-1f, 0x1.5fd384p-1f, 0x1.058672p-1f);
 }
 
 // bs_exp_half_sq, lane for lane (-x as a sign flip, exact).
