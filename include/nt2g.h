@@ -500,7 +500,7 @@ typedef struct nt2g_batch_item {
 typedef struct nt2g_batch_tune {
     int32_t block_threads;     /* 128..1024, multiple of 32 */
     int32_t blocks_per_sm;     /* resident blocks per SM of the persistent grid */
-    int32_t tile_vectors;      /* float4 vectors per tile per thread */
+    int32_t tile_vectors;      /* float4 vectors per tile per thread (0: 1 to 8, by the total size) */
     int32_t precision;         /* nt2g_precision */
     int32_t vector_width;      /* float4 vectors a thread has in flight per step: 1 or 2 (0 = 1) */
     int32_t reserved;
