@@ -102,10 +102,7 @@ __device__ __forceinline__ void run_tile(const DItem &it, int64_t start, int64_t
     default: {
         const float4 *X = (const float4 *)it.in[0], *Y = (const float4 *)it.in[1], *Z = (const float4 *)it.in[2];
         auto one = [&](const float4 x, const float4 y, const float4 z, int64_t at) {
-            float4 o;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) set(o, j, expr3_elem<P>(get(x, j), get(y, j), get(z, j)));
-            st_stream((float4 *)it.out[0] + at, o);
+            st_stream((float4 *)it.out[0] + at, expr3_vec4<P>(x, y, z));
         };
         if constexpr (VW == 2)
             for (; i + bd < v1; i += 2 * bd) {

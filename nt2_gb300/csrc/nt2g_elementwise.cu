@@ -5,6 +5,7 @@
 #include <string.h>
 #include "nt2g_common.cuh"
 #include "nt2g_exprs.cuh"
+#include "nt2g_pair.cuh"
 #include "nt2g_internal.h"
 
 namespace nt2g {
@@ -75,10 +76,8 @@ __global__ void __launch_bounds__(kThreads) k_expr3(const float *__restrict__ x,
         const int64_t nv = n >> 2;
         for (int64_t i = tid; i < nv; i += stride) {
             float4 a = ld_stream((const float4 *)x + i), b = ld_stream((const float4 *)y + i),
-                   c = ld_stream((const float4 *)z + i), r;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) set(r, j, expr3_elem<P>(get(a, j), get(b, j), get(c, j)));
-            st_stream((float4 *)o + i, r);
+                   c = ld_stream((const float4 *)z + i);
+            st_stream((float4 *)o + i, expr3_vec4<P>(a, b, c));
         }
         done = nv << 2;
     }

@@ -183,6 +183,7 @@ static const char *lane_function(int code)
     switch (code) {
     case NT2G_OP_EXP: return "exp";
     case NT2G_OP_LOG: return "log";
+    case NT2G_OP_LOG1P: return "log1p";
     case NT2G_OP_SIN: return "sin";
     case NT2G_OP_COS: return "cos";
     case NT2G_OP_POW: return "pow";

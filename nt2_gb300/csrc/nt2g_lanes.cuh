@@ -6,9 +6,10 @@
 // common range each lane performs exactly the operations of the scalar
 // function of nt2g_math.cuh, so both give the same bits, and the interpreter,
 // which evaluates one lane at a time, agrees with the compiled kernels.
-// What bounds these kernels is instruction issue: a select or a compare per
-// special value and lane was a third of it, packed arithmetic halves another.
-// TODO figures
+// What bounds these kernels is instruction issue: compares and selects per
+// special value and lane were a third of it, packed arithmetic halves another
+// (2^24 elements of sin(x) cos(y), pow(x, y) and erf(y) + gammaln(x) in one tie:
+// 220 us one lane at a time, 142 so).
 // Also compiled by NVRTC (the run-time source puts nt2g_math.cuh and
 // nt2g_f2.cuh ahead of it).
 #pragma once
@@ -146,6 +147,44 @@ template <class P, int L, int A> __device__ __forceinline__ void log(const float
     NT2G_LANES_HEAD(r[j] = nt2g::log<P>(a[j]), !positive_normal(a[j]))
 #pragma unroll
     for (int j = 0; j + 1 < L; j += 2) upk(log_pos_fast2(pk(a[j], a[j + 1])), r[j], r[j + 1]);
+}
+
+// log1p where u = 1 + a is a positive normal number; the quotient of u's
+// rounding error by u correctly rounded (Markstein: q + (c - q u) y with y the
+// correctly rounded 1/u; c is 0 or at least 2^-49 where u != 1, so no step
+// underflows; u = 1 divides exactly, and above 2^25 c is 0)
+__device__ __forceinline__ f2 log1p2(f2 a, f2 u)
+{
+    const f2 c = sub2(a, sub2(u, dup(1.0f))), y = recip_rn2(u), nu = negx2(u);
+    const f2 q = mul2(c, y);
+    return add2(log_pos_fast2(u), fma2(fma2(nu, q, c), y, q));
+}
+template <class P, int L, int A> __device__ __forceinline__ void log1p(const float (&a)[A], float (&r)[A])
+{
+    NT2G_LANES_HEAD(r[j] = nt2g::log1p<P>(a[j]), !positive_normal(Fast::add(1.0f, a[j])))
+#pragma unroll
+    for (int j = 0; j + 1 < L; j += 2) {
+        const f2 x = pk(a[j], a[j + 1]);
+        upk(log1p2(x, add2(dup(1.0f), x)), r[j], r[j + 1]);
+    }
+}
+
+// exp(-x^2): exp_neg_sqr lane for lane
+template <class P, int L, int A> __device__ __forceinline__ void exp_neg_sqr(const float (&a)[A], float (&r)[A])
+{
+    NT2G_LANES_HEAD(r[j] = nt2g::exp_neg_sqr<P>(a[j]), is_nan(a[j]))
+#pragma unroll
+    for (int j = 0; j + 1 < L; j += 2) {
+        const f2 x = pk(a[j], a[j + 1]), hi = mul2(x, x), nhi = negx2(hi), nlo = negx2(fma2(x, x, nhi));
+        f2 scale;
+        f2 s = exp_parts2(nhi, scale);
+        s = add2(s, fma2(nlo, s, nlo));
+        float r0, r1, h0, h1;
+        upk(mul2(add2(s, dup(1.0f)), scale), r0, r1);
+        upk(nhi, h0, h1);
+        r[j] = h0 <= bits_f(NT2G_MINLOG) ? 0.0f : r0;
+        r[j + 1] = h1 <= bits_f(NT2G_MINLOG) ? 0.0f : r1;
+    }
 }
 
 template <class P, int L, int A>
