@@ -38,6 +38,7 @@ constexpr int64_t kSmallSeg = 64;        // (many) segments up to this length: o
 // A table as a fold source: streaming loads.
 struct RawSrc {
     static constexpr int kBatch = 4;  // vectors a thread has in flight
+    static constexpr bool kAsync = true;
     const float *x;
     typedef float4 Raw;
     __device__ __forceinline__ float at(int64_t pos) const { return ld_stream(x + pos); }

@@ -527,6 +527,50 @@ template <bool MX, int W> __device__ __forceinline__ Best lanes_best(Best a, uns
     return a;
 }
 
+// ---------------------------------------------------- a thread's own ring --
+// A table's vectors go through shared memory, where a thread's next kRing of
+// them wait without holding registers: S at a time, each thread its own slots,
+// so there is nothing to synchronise.  (Loads into registers were in flight
+// only between one batch's arithmetic and the next.  6000 x 8192, along either
+// dimension: variances 56 us then, 55 and 52 now, which leaves their two dozen
+// operations a pair; means 35, now 33; maxima along rows 45, now 40.)
+constexpr int kRing = 8;
+__device__ __forceinline__ void ring_copy(float4 *to, const float *from)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(to)), "l"(from)
+                 : "memory");
+}
+// take(e, n, r): the thread's rows r .. r + n of `rows`, `stride` floats apart
+// from `at` on, as e[u][0..4)
+template <int S, class Take>
+__device__ __forceinline__ void ring_rows(float4 *ring, const float *at, int64_t stride, int rows, Take take)
+{
+    constexpr int R = kRing / S;
+    float4 *const mine = ring + threadIdx.x;
+    auto fill = [&](int s) {
+#pragma unroll
+        for (int u = 0; u < S; ++u) {
+            if (s * S + u < rows) ring_copy(mine + ((s & (R - 1)) * S + u) * kThreads, at);
+            at += stride;
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+#pragma unroll
+    for (int s = 0; s < R; ++s) fill(s);
+    for (int s = 0; s * S < rows; ++s) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(R - 1) : "memory");
+        float e[S][4];
+#pragma unroll
+        for (int u = 0; u < S; ++u) {
+            const float4 v = mine[((s & (R - 1)) * S + u) * kThreads];
+            e[u][0] = v.x; e[u][1] = v.y; e[u][2] = v.z; e[u][3] = v.w;
+        }
+        if (rows - s * S >= S) take(e, S, s * S);
+        else take(e, rows - s * S, s * S);
+        fill(s + R);  // (the slot just read)
+    }
+}
+
 // ----------------------------------------- contiguous segments (lo == 1) --
 // G threads (8, 32 or the block's 256) per (segment, chunk) work item, a few
 // items a block one after the other: a segment's loads are in flight at once
@@ -545,6 +589,8 @@ __device__ __forceinline__ void inner_body(const Src &src, int64_t inner, int64_
     constexpr bool MX = OP == MAX, EXT = OP == MAX || OP == MIN;
     constexpr int W = G < 32 ? G : 32, kGroups = kThreads / G, kWarps = kThreads / 32;
     constexpr int kBatch = Src::kBatch;
+    constexpr bool kAsync = Src::kAsync && !EXT;  // (extremes look at a batch of all lanes)
+    __shared__ float4 s_ring[kAsync ? kRing * kThreads : 1];
     __shared__ Partial s_item[FINAL ? kItems : 1];
     __shared__ Partial s_warp[2][kWarps];
     __shared__ float s_mean;
@@ -590,24 +636,30 @@ __device__ __forceinline__ void inner_body(const Src &src, int64_t inner, int64_
         auto sweep = [&]() {
             if (vec) {
                 const int64_t a = (p0 + 3) >> 2, b = p1 >> 2;  // whole vectors [a, b)
-                for (int64_t j = a; j < b; j += kBatch * G) {
-                    const int64_t left = b - j - tid;
-                    float e[kBatch][4];
-                    typename Src::Raw raw[kBatch];
-                    const int n = left <= 0 ? 0 : left > (kBatch - 1) * G ? kBatch : (int)((left + G - 1) / G);
-#pragma unroll
-                    for (int u = 0; u < kBatch; ++u) {  // (past the end: the last one again, so that no load waits for a branch)
-                        const int64_t at = j + tid + u * G;
-                        raw[u] = src.fetch4(4 * (at < b ? at : b - 1));
+                if constexpr (kAsync) {
+                    const int64_t left = b - a - tid;
+                    ring_rows<2>(s_ring, src.x + 4 * (a + tid), 4 * G, left > 0 ? (int)((left + G - 1) / G) : 0,
+                                 [&](const float(&e)[2][4], int n, int) { take(e, n, 0, 0); });
+                } else {
+                    for (int64_t j = a; j < b; j += kBatch * G) {
+                        const int64_t left = b - j - tid;
+                        float e[kBatch][4];
+                        typename Src::Raw raw[kBatch];
+                        const int n = left <= 0 ? 0 : left > (kBatch - 1) * G ? kBatch : (int)((left + G - 1) / G);
+    #pragma unroll
+                        for (int u = 0; u < kBatch; ++u) {  // (past the end: the last one again, so that no load waits for a branch)
+                            const int64_t at = j + tid + u * G;
+                            raw[u] = src.fetch4(4 * (at < b ? at : b - 1));
+                        }
+    #pragma unroll
+                        for (int u = 0; u < kBatch; ++u) {
+                            const int64_t at = j + tid + u * G;
+                            src.value4(raw[u], 4 * (at < b ? at : b - 1), e[u]);
+                        }
+                        const int32_t pos = (int32_t)(4 * (j + tid) - p0);
+                        if (j + kBatch * G <= b) take(e, kBatch, pos, 4 * G);
+                        else take(e, n, pos, 4 * G);
                     }
-#pragma unroll
-                    for (int u = 0; u < kBatch; ++u) {
-                        const int64_t at = j + tid + u * G;
-                        src.value4(raw[u], 4 * (at < b ? at : b - 1), e[u]);
-                    }
-                    const int32_t pos = (int32_t)(4 * (j + tid) - p0);
-                    if (j + kBatch * G <= b) take(e, kBatch, pos, 4 * G);
-                    else take(e, n, pos, 4 * G);
                 }
                 // up to three elements on either side
                 const int64_t first = 4 * a < p1 ? 4 * a : p1, last = 4 * b > first ? 4 * b : first;
@@ -762,6 +814,12 @@ __device__ __forceinline__ void outer_body(const Src &src, int64_t lo, int64_t i
 {
     constexpr bool MX = OP == MAX, EXT = OP == MAX || OP == MIN;
     constexpr int kWarps = kThreads / 32, kRows = Src::kBatch;
+    constexpr bool kAsync = Src::kAsync && VEC == 4;
+    // the rings, and then in their place the warps' partials
+    constexpr int kPartBytes = kWarps * 32 * VEC * (int)sizeof(Partial), kRingBytes = kAsync ? kRing * kThreads * 16 : 0;
+    __shared__ __align__(16) char s_mem[kPartBytes > kRingBytes ? kPartBytes : kRingBytes];
+    float4 *const s_ring = (float4 *)s_mem;
+    Partial(*const s_part)[32 * VEC] = (Partial(*)[32 * VEC])s_mem;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int64_t lv = lo / VEC;  // thread columns per h
     const int64_t c = blockIdx.y;
@@ -789,8 +847,8 @@ __device__ __forceinline__ void outer_body(const Src &src, int64_t lo, int64_t i
             if constexpr (VEC == 4) src.value4(r, base + lo * k, e);
             else e[0] = src.value(r, base + lo * k);
         };
-        // rows k, k + kWarps, ...
-        auto take = [&](const auto &e, int64_t k) {
+        // n rows k, k + kWarps, ...
+        auto take = [&](const auto &e, int n, int64_t k) {
             constexpr int U = sizeof(e) / sizeof(e[0]);
             if constexpr (EXT) {
 #pragma unroll
@@ -798,11 +856,12 @@ __device__ __forceinline__ void outer_body(const Src &src, int64_t lo, int64_t i
                     float col[U][1];
 #pragma unroll
                     for (int u = 0; u < U; ++u) col[u][0] = e[u][v];
-                    run[v].batch(col, U, (int32_t)(k - k0), kWarps, 0);
+                    run[v].batch(col, n, (int32_t)(k - k0), kWarps, 0);
                 }
             } else {
 #pragma unroll
-                for (int u = 0; u < U; ++u)
+                for (int u = 0; u < U; ++u) {
+                    if (u >= n) break;
 #pragma unroll
                     for (int v = 0; v < VEC; ++v) {
                         if constexpr (is_var(OP)) {  // (VEC == 1: both halves the same)
@@ -813,9 +872,17 @@ __device__ __forceinline__ void outer_body(const Src &src, int64_t lo, int64_t i
                             sum_elem_c<OP>(acc[v], e[u][v], m[v], md[v]);
                         }
                     }
+                }
             }
         };
         auto sweep = [&]() {
+            if constexpr (kAsync) {
+                const int64_t left = k1 - k0 - wid;
+                ring_rows<EXT ? 4 : 2>(s_ring, src.x + base + lo * (k0 + wid), lo * kWarps,
+                                       left > 0 ? (int)((left + kWarps - 1) / kWarps) : 0,
+                                       [&](const auto &e, int n, int r) { take(e, n, k0 + wid + r * kWarps); });
+                return;
+            }
             int64_t k = k0 + wid;
             for (; k + (kRows - 1) * kWarps < k1; k += kRows * kWarps) {
                 float e[kRows][VEC];
@@ -824,12 +891,12 @@ __device__ __forceinline__ void outer_body(const Src &src, int64_t lo, int64_t i
                 for (int u = 0; u < kRows; ++u) raw[u] = fetch(k + u * kWarps);
 #pragma unroll
                 for (int u = 0; u < kRows; ++u) value(raw[u], k + u * kWarps, e[u]);
-                take(e, k);
+                take(e, kRows, k);
             }
             for (; k < k1; k += kWarps) {
                 float e[1][VEC];
                 value(fetch(k), k, e[0]);
-                take(e, k);
+                take(e, 1, k);
             }
         };
 #pragma unroll
@@ -845,8 +912,8 @@ __device__ __forceinline__ void outer_body(const Src &src, int64_t lo, int64_t i
         }
         if (live) sweep();
         // warps combine: thread i finishes output i of the block's
-        __shared__ Partial s_part[kWarps][32 * VEC];
         auto give = [&]() {
+            if constexpr (kAsync) __syncthreads();  // (the partials take the rings' place)
 #pragma unroll
             for (int v = 0; v < VEC; ++v) {
                 Partial &r = s_part[wid][lane * VEC + v];

@@ -478,7 +478,7 @@ std::string jit_fold_source(const std::vector<nt2g_op> &ops, const std::vector<u
     int tables = 0;
     for (const nt2g_op &o : ops) tables += o.code == NT2G_OP_LOAD;
     s += "struct ExprSrc {\n    static constexpr int kBatch = " + std::string(tables <= 1 ? "4" : "2") +
-         ";\n    JitArgs a;\n"
+         ";\n    static constexpr bool kAsync = false;\n    JitArgs a;\n"
          "    typedef JitIn Raw;\n"
          "    __device__ __forceinline__ Raw fetch(long long pos) const { Raw r; jit_fetch<false>(a, pos, 1, r); return r; }\n"
          "    __device__ __forceinline__ Raw fetch4(long long pos) const { Raw r; jit_fetch<true>(a, pos, 4, r); return r; }\n"
