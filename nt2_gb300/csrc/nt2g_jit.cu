@@ -1294,8 +1294,13 @@ nt2g_status launch_jit(const std::vector<nt2g_op> &ops, const std::vector<uint8_
     for (int s = 0; s < kMaxSlots; ++s)
         if (args.ptr[s]) vec &= ((uintptr_t)args.ptr[s] & (args.dtype[s] == NT2G_F32 ? 15u : 3u)) == 0;
     int64_t full = (int64_t)device_sm_count() * (e->blocks_per_sm > 0 ? e->blocks_per_sm : 1);
-    int64_t need = (count + 1023) / 1024;  // 256 threads x 4 elements
-    int grid = (int)(need < full ? need : full);
+    const int64_t need = (count + 1023) / 1024;  // 256 threads x 4 elements
+    // four waves of blocks rather than one that strides over everything: SMs do
+    // not finish alike, and blocks that come later fill those done first (2^24
+    // elements of three functor programs: 142 us, 136 with two waves, 133 with
+    // four or eight, 135 with a block for every 1024 elements)
+    full *= 4;
+    const int grid = (int)(need < full ? need : full);
     long long n = count;
     void *params[] = {(void *)&args, (void *)&n, (void *)&vec};
     cudaError_t ce = cudaLaunchKernel((const void *)e->kernel, dim3(grid), dim3(256), params, 0, st);

@@ -373,28 +373,32 @@ template <class P, int L, int A> __device__ __forceinline__ void gammaln(const f
     if (small)
 #pragma unroll
         for (int j = 0; j + 1 < L; j += 2) {
+            // The steps towards (1.5, 2.5]: down by 1 to 4 from above 2.5 (exact
+            // subtractions), up by 1 or 2 from below 1.5.  The products of all the
+            // steps are at hand after four multiplications, and each comparison
+            // picks the product and the shift of one more step.
             const f2 x = pk(a[j], a[j + 1]), one = dup(1.0f);
-            float t[2] = {a[j], a[j + 1]}, z[2] = {1.0f, 1.0f}, nx[2] = {0.0f, 0.0f};
+            const f2 d1 = sub2(x, one), d2 = mul2(d1, sub2(x, dup(2.0f))), d3 = mul2(d2, sub2(x, dup(3.0f))),
+                     d4 = mul2(d3, sub2(x, dup(4.0f))), u1 = add2(x, one), u2 = mul2(x, u1);
+            float z[2], nx[2], d1_[2], d2_[2], d3_[2], d4_[2], u1_[2], u2_[2];
+            upk(d1, d1_[0], d1_[1]);
+            upk(d2, d2_[0], d2_[1]);
+            upk(d3, d3_[0], d3_[1]);
+            upk(d4, d4_[0], d4_[1]);
+            upk(u1, u1_[0], u1_[1]);
+            upk(u2, u2_[0], u2_[1]);
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const f2 n = pk(nx[0], nx[1]), tt = pk(t[0], t[1]), zz = pk(z[0], z[1]);
-                const f2 nd = sub2(n, one), td = add2(x, nd), nu = add2(n, one), tu = add2(x, nu);
-                float nd_[2], td_[2], nu_[2], tu_[2], zd[2], zu[2];
-                upk(nd, nd_[0], nd_[1]);
-                upk(td, td_[0], td_[1]);
-                upk(nu, nu_[0], nu_[1]);
-                upk(tu, tu_[0], tu_[1]);
-                upk(mul2(zz, td), zd[0], zd[1]);
-                upk(mul2(zz, tt), zu[0], zu[1]);
-#pragma unroll
-                for (int i = 0; i < 2; ++i) {
-                    const bool dn = t[i] > 2.5f, up = t[i] < 1.5f;
-                    z[i] = dn ? zd[i] : up ? zu[i] : z[i];
-                    nx[i] = dn ? nd_[i] : up ? nu_[i] : nx[i];
-                    t[i] = dn ? td_[i] : up ? tu_[i] : t[i];
-                }
+            for (int i = 0; i < 2; ++i) {
+                const float v = a[j + i];
+                z[i] = 1.0f, nx[i] = -2.0f;
+                if (v < 1.5f) z[i] = v, nx[i] = -1.0f;
+                if (u1_[i] < 1.5f) z[i] = u2_[i], nx[i] = 0.0f;
+                if (v > 2.5f) z[i] = d1_[i], nx[i] = -3.0f;
+                if (v > 3.5f) z[i] = d2_[i], nx[i] = -4.0f;
+                if (v > 4.5f) z[i] = d3_[i], nx[i] = -5.0f;
+                if (v > 5.5f) z[i] = d4_[i], nx[i] = -6.0f;
             }
-            const f2 xb = add2(x, sub2(pk(nx[0], nx[1]), dup(2.0f)));
+            const f2 xb = add2(x, pk(nx[0], nx[1]));
             float lz[2];
             upk(log_pos_fast2(pk(z[0], z[1])), lz[0], lz[1]);
             const f2 gb = horner2(xb, dup(bits_f(0x3a1ebb94u)), bits_f(0xbaabeab1u), bits_f(0x3b3ba883u), bits_f(0xbbf164fdu),
