@@ -103,6 +103,10 @@ template <bool FULL> __device__ __forceinline__ void jit_ldf(float (&d)[2], cons
     if (FULL) { const float2 t = __ldcs((const float2 *)q); d[0] = t.x; d[1] = t.y; }
     else { d[0] = q[0]; d[1] = cnt > 1 ? q[1] : 0.0f; }
 }
+__device__ __forceinline__ void jit_copy8(void *to, const float *from)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(to)), "l"(from) : "memory");
+}
 template <bool FULL> __device__ __forceinline__ void jit_stf(void *p, long long i, int cnt, const float (&v)[2])
 {
     float *q = (float *)p + i;
@@ -828,6 +832,13 @@ std::vector<int> vjp_scalar_slots(const std::vector<nt2g_op> &ops, const std::ve
     return slots;
 }
 
+// A thread's next elements wait in its own slots of shared memory (one pair of
+// each table ahead), so their loads run beside the arithmetic without holding
+// registers (2^24 options' reverse mode: 174 us, stalled on loads in half of
+// its cycles, without; 167 with); programs of more than kVjpRing tables load
+// directly.
+constexpr size_t kVjpRing = 8;  // 2 x 8 x 256 x 8 bytes: 32 KB
+
 // The reverse-mode kernel of a program: each thread recomputes the forward
 // values of 4 consecutive elements (the statements of jit_source, so the
 // same bits as nt2g_eval), seeds the adjoints of the values stored into each
@@ -851,21 +862,58 @@ std::string jit_vjp_source(const std::vector<nt2g_op> &ops, const std::vector<ui
     s += kJitPrelude;
     s += "struct VjpArgs { const float *ct[16]; float *grad[16]; };\n";
     s += "#define NT2G_NS " + std::to_string(ns > 0 ? ns : 1) + "\n";
-    s += "template <class P, bool FULL>\n__device__ __forceinline__ void vjp_tile(const JitArgs &a, const VjpArgs &g, "
-         "long long i, int cnt, nt2g::CSum (&sacc)[NT2G_NS])\n{\n    typedef nt2g::Fast D;\n    constexpr int L = 2, A = 2;\n";
-    emit_body(s, ops, logical, false);
-    for (size_t k = 0; k < ops.size(); ++k)
-        if (act[k]) s += "    float g" + std::to_string(k) + "[A] = {0.0f, 0.0f};\n";
-    // seeds: the cotangent of each output slot flows into the last value stored there
+    // what a tile reads: its tables and the cotangents of its outputs
     std::vector<int> last_store(kMaxSlots, -1);
     for (size_t k = 0; k < ops.size(); ++k)
         if (ops[k].code == NT2G_OP_STORE) last_store[ops[k].b] = (int)k;
+    struct Row { std::string to, from; bool optional; };
+    std::vector<Row> rows;
+    std::string members, bytes;
+    for (size_t k = 0; k < ops.size(); ++k) {
+        if (ops[k].code != NT2G_OP_LOAD) continue;
+        const std::string v = "v" + std::to_string(k), from = "a.ptr[" + std::to_string(ops[k].a) + "]";
+        members += (ops[k].dtype == NT2G_F32 ? " float " : " unsigned ") + v + "[2];";
+        if (ops[k].dtype == NT2G_F32) rows.push_back({v, from, false});
+        else bytes += "    jit_ldb<FULL>(in." + v + ", " + from + ", i, cnt);\n";
+    }
+    for (int slot = 0; slot < kMaxSlots; ++slot)
+        if (last_store[slot] >= 0 && act[ops[last_store[slot]].a]) {
+            const std::string sl = std::to_string(slot);
+            members += " float c" + sl + "[2];";
+            rows.push_back({"c" + sl, "g.ct[" + sl + "]", true});
+        }
+    const bool ring = !rows.empty() && rows.size() <= kVjpRing;
+    s += "struct JitIn {" + members + " char none; };\n";
+    s += "template <bool FULL>\n__device__ __forceinline__ void jit_bytes(const JitArgs &a, long long i, int cnt, JitIn &in)\n{\n" +
+         bytes + "}\ntemplate <bool FULL>\n__device__ __forceinline__ void jit_fetch(const JitArgs &a, const VjpArgs &g, long long i, "
+         "int cnt, JitIn &in)\n{\n";
+    for (const Row &r : rows)
+        s += std::string(r.optional ? "    if (" + r.from + ") " : "    ") + "jit_ldf<FULL>(in." + r.to + ", " + r.from + ", i, cnt);\n";
+    s += "    jit_bytes<FULL>(a, i, cnt, in);\n}\n";
+    if (ring) {
+        s += "__device__ __forceinline__ void ring_fill(float2 (&r)[" + std::to_string(rows.size()) +
+             "][256], const JitArgs &a, const VjpArgs &g, long long i, long long n)\n{\n    if (i + 2 <= n) {\n";
+        for (size_t q = 0; q < rows.size(); ++q)
+            s += "    " + std::string(rows[q].optional ? "    if (" + rows[q].from + ") " : "    ") + "jit_copy8(&r[" + std::to_string(q) +
+                 "][threadIdx.x], (const float *)" + rows[q].from + " + i);\n";
+        s += "    }\n    asm volatile(\"cp.async.commit_group;\" ::: \"memory\");\n}\n"
+             "__device__ __forceinline__ void ring_read(const float2 (&r)[" + std::to_string(rows.size()) + "][256], JitIn &in)\n{\n";
+        for (size_t q = 0; q < rows.size(); ++q)
+            s += "    { const float2 t = r[" + std::to_string(q) + "][threadIdx.x]; in." + rows[q].to + "[0] = t.x; in." + rows[q].to +
+                 "[1] = t.y; }\n";
+        s += "}\n";
+    }
+    s += "template <class P, bool FULL>\n__device__ __forceinline__ void vjp_tile(const JitArgs &a, const VjpArgs &g, "
+         "const JitIn &in, long long i, int cnt, nt2g::CSum (&sacc)[NT2G_NS])\n{\n    typedef nt2g::Fast D;\n    constexpr int L = 2, A = 2;\n";
+    emit_body(s, ops, logical, false, true);
+    for (size_t k = 0; k < ops.size(); ++k)
+        if (act[k]) s += "    float g" + std::to_string(k) + "[A] = {0.0f, 0.0f};\n";
+    // seeds: the cotangent of each output slot flows into the last value stored there
     for (int slot = 0; slot < kMaxSlots; ++slot) {
         const int st = last_store[slot];
         if (st < 0 || !act[ops[st].a]) continue;
         const std::string sl = std::to_string(slot), val = std::to_string(ops[st].a);
-        s += "    if (g.ct[" + sl + "]) { float t[A]; jit_ldf<FULL>(t, g.ct[" + sl + "], i, cnt); NT2G_LL g" + val +
-             "[j] += t[j]; }\n";
+        s += "    if (g.ct[" + sl + "]) { NT2G_LL g" + val + "[j] += in.c" + sl + "[j]; }\n";
     }
     std::vector<uint8_t> phi_done(ops.size(), 0);
     for (size_t k = ops.size(); k-- > 0;) {
@@ -907,10 +955,32 @@ std::string jit_vjp_source(const std::vector<nt2g_op> &ops, const std::vector<ui
     s += "    nt2g::CSum sacc[NT2G_NS];\n"
          "    for (int q = 0; q < NT2G_NS; ++q) sacc[q] = nt2g::CSum{0.0f, 0.0f};\n"
          "    const long long stride = (long long)gridDim.x * blockDim.x * 2;\n"
-         "    for (long long i = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * 2; i < n; i += stride) {\n"
+         "    long long i = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * 2;\n";
+    if (ring)
+        s += "    if (vec) {\n"
+             "        __shared__ float2 r[2][" + std::to_string(rows.size()) + "][256];\n"
+             "        ring_fill(r[0], a, g, i, n);\n"
+             "        ring_fill(r[1], a, g, i + stride, n);\n"
+             "        for (int t = 0; i + 2 <= n; i += stride, t ^= 1) {\n"
+             "            asm volatile(\"cp.async.wait_group 1;\" ::: \"memory\");\n"
+             "            JitIn in;\n"
+             "            ring_read(r[t], in);\n"
+             "            jit_bytes<true>(a, i, 2, in);\n"
+             "            vjp_tile<P, true>(a, g, in, i, 2, sacc);\n"
+             "            ring_fill(r[t], a, g, i + 2 * stride, n);\n"
+             "        }\n"
+             "    }\n";
+    s += "    for (; i < n; i += stride) {\n"
          "        const int cnt = n - i < 2 ? (int)(n - i) : 2;\n"
-         "        if (vec && cnt == 2) vjp_tile<P, true>(a, g, i, 2, sacc);\n"
-         "        else vjp_tile<P, false>(a, g, i, cnt, sacc);\n"
+         "        JitIn in;\n";
+    if (!ring)
+        s += "        if (vec && cnt == 2) {\n"
+             "            jit_fetch<true>(a, g, i, 2, in);\n"
+             "            vjp_tile<P, true>(a, g, in, i, 2, sacc);\n"
+             "            continue;\n"
+             "        }\n";
+    s += "        jit_fetch<false>(a, g, i, cnt, in);\n"
+         "        vjp_tile<P, false>(a, g, in, i, cnt, sacc);\n"
          "    }\n";
     if (ns > 0)
         s += "    __shared__ double red[8][NT2G_NS];\n"
@@ -1225,6 +1295,10 @@ nt2g_status launch_vjp(const std::vector<nt2g_op> &ops, const std::vector<uint8_
     const int ns = (int)sslots.size();
     const int64_t bound = vjp_grid_bound(count);
     int64_t full = (int64_t)device_sm_count() * (e->blocks_per_sm > 0 ? e->blocks_per_sm : 1);
+    // a second wave fills the SMs that finish first, where a thread still has eight
+    // pairs or more (2^24 elements: 167 us with one wave, 162 with two; 2^20: 14.0
+    // and 15.3, the blocks' scalar sums included)
+    if (count >= full * 2 * 256 * 2 * 8) full *= 2;
     const int grid = (int)(bound < full ? bound : full);
     double *partials = nullptr;
     if (scalar_grads && ns > 0) {
@@ -1298,8 +1372,10 @@ nt2g_status launch_jit(const std::vector<nt2g_op> &ops, const std::vector<uint8_
     // four waves of blocks rather than one that strides over everything: SMs do
     // not finish alike, and blocks that come later fill those done first (2^24
     // elements of three functor programs: 142 us, 136 with two waves, 133 with
-    // four or eight, 135 with a block for every 1024 elements)
-    full *= 4;
+    // four or eight, 135 with a block for every 1024 elements).  Not where that
+    // leaves a thread a vector or two, which a block's start costs as much as it
+    // gives (2^20 elements under the NT2 policy: 44.1 us in one wave, 45.1).
+    if (need >= 4 * full) full *= 4;
     const int grid = (int)(need < full ? need : full);
     long long n = count;
     void *params[] = {(void *)&args, (void *)&n, (void *)&vec};
