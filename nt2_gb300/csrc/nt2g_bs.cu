@@ -57,7 +57,7 @@ __device__ unsigned long long g_bs_wait_timeouts = 0;
 
 // Pipelined form for aligned tables: a persistent grid walks tiles of 1024
 // options (one float4 per thread of a 256-thread block).  Thread 0 keeps the
-// block's next STAGES - 1 tiles of S, K, T (and sigma) in flight as bulk
+// block's next STAGES - 1 tiles of S, K, T and sigma in flight as bulk
 // copies into shared memory, each stage completing on its mbarrier, so the
 // loads of later tiles overlap the pricing of the current one and no warp
 // waits on HBM latency once the pipeline is primed.  Results go straight to
@@ -65,26 +65,24 @@ __device__ unsigned long long g_bs_wait_timeouts = 0;
 // it every thread has read the previous stage, which thread 0 then refills.
 // The options past the last whole tile (fewer than 1024) are priced by block
 // 0 with plain loads.
-template <class P, bool SIG_TAB, int STAGES>
-__global__ void __launch_bounds__(256, SIG_TAB ? 4 : 5) k_bs_pipe(const float *__restrict__ S, const float *__restrict__ K,
-                                                 const float *__restrict__ T, const float *__restrict__ sig,
-                                                 float sig_s, float r, float *__restrict__ call,
-                                                 float *__restrict__ put, int64_t n)
+template <int STAGES>
+__global__ void __launch_bounds__(256, 4) k_bs_pipe(const float *__restrict__ S, const float *__restrict__ K,
+                                                    const float *__restrict__ T, const float *__restrict__ sig, float r,
+                                                    float *__restrict__ call, float *__restrict__ put, int64_t n)
 {
-    constexpr int NT = SIG_TAB ? 4 : 3;  // tables per tile
+    constexpr int NT = 4;                // tables per tile
     constexpr int TILE = 1024;           // options per tile
     constexpr uint32_t TILE_BYTES = TILE * 4;
     extern __shared__ __align__(128) float4 stage_buf[];  // [STAGES][NT][256]
     uint64_t *full = reinterpret_cast<uint64_t *>(stage_buf + STAGES * NT * 256);
     const int tid = threadIdx.x;
     const int64_t ntiles = n / TILE, G = gridDim.x;
-    const float inv_sig_s = P::exact || SIG_TAB ? 0.0f : inv_fast(sig_s);
     auto issue = [&](int s, int64_t t) {
         mbar_arrive_expect_tx(&full[s], NT * TILE_BYTES);
         bulk_copy_g2s(stage_buf + (s * NT + 0) * 256, S + t * TILE, TILE_BYTES, &full[s]);
         bulk_copy_g2s(stage_buf + (s * NT + 1) * 256, K + t * TILE, TILE_BYTES, &full[s]);
         bulk_copy_g2s(stage_buf + (s * NT + 2) * 256, T + t * TILE, TILE_BYTES, &full[s]);
-        if (SIG_TAB) bulk_copy_g2s(stage_buf + (s * NT + 3) * 256, sig + t * TILE, TILE_BYTES, &full[s]);
+        bulk_copy_g2s(stage_buf + (s * NT + 3) * 256, sig + t * TILE, TILE_BYTES, &full[s]);
     };
     if (tid == 0) {
         for (int s = 0; s < STAGES; ++s) mbar_init(&full[s], 1);
@@ -114,10 +112,9 @@ __global__ void __launch_bounds__(256, SIG_TAB ? 4 : 5) k_bs_pipe(const float *_
             issue((int)((it - 1) % STAGES), t + (STAGES - 1) * G);
         }
         const float4 sv = stage_buf[(s * NT + 0) * 256 + tid], kv = stage_buf[(s * NT + 1) * 256 + tid],
-                     tv = stage_buf[(s * NT + 2) * 256 + tid];
-        const float4 vv = SIG_TAB ? stage_buf[(s * NT + 3) * 256 + tid] : make_float4(sig_s, sig_s, sig_s, sig_s);
+                     tv = stage_buf[(s * NT + 2) * 256 + tid], vv = stage_buf[(s * NT + 3) * 256 + tid];
         float4 c, p;
-        bs_compute4<P, SIG_TAB>(sv, kv, tv, vv, inv_sig_s, r, c, p);
+        bs_compute4<Fast, true>(sv, kv, tv, vv, 0.0f, r, c, p);
         const int64_t o = t * 256 + tid;
         st_stream((float4 *)call + o, c);
         st_stream((float4 *)put + o, p);
@@ -125,11 +122,10 @@ __global__ void __launch_bounds__(256, SIG_TAB ? 4 : 5) k_bs_pipe(const float *_
     if (blockIdx.x == 0) {
         const int64_t nv = n >> 2;
         for (int64_t i = ntiles * 256 + tid; i < nv; i += blockDim.x)
-            bs_float4<P, SIG_TAB>(S, K, T, sig, sig_s, inv_sig_s, r, call, put, i);
+            bs_float4<Fast, true>(S, K, T, sig, 0.0f, 0.0f, r, call, put, i);
         if (tid < (n & 3)) {
             const int64_t i = (nv << 2) + tid;
-            const float sj = SIG_TAB ? sig[i] : sig_s;
-            bs_option<P>(S[i], K[i], T[i], sj, SIG_TAB ? inv_fast(sj) : inv_sig_s, r, call[i], put[i]);
+            bs_option<Fast>(S[i], K[i], T[i], sig[i], inv_fast(sig[i]), r, call[i], put[i]);
         }
     }
 }
@@ -375,29 +371,28 @@ static int grid_for(KERN k, int64_t n)
     return persistent_blocks(k, 256, 0, 256 * 4, n);
 }
 
-// The pipelined kernel takes aligned batches from 2^22 options on: it keeps
-// bulk copies of three tiles per block in flight, which matches the
-// one-float4-per-thread kernel's throughput there (both are issue-bound at
-// ~98 instructions per option) while reading HBM through the copy engine;
-// below it the persistent grid's ramp costs more than it saves.
+// The pipelined kernel takes the fast policy's options with a volatility table
+// from 2^22 aligned ones on: there four loads an option wait longer than its
+// arithmetic hides (2^24 options: 80 us one float4 a thread, 74 in one wave of
+// pipelined blocks, 72 in two).  Everywhere else both kernels wait for the
+// arithmetic, and blocks that leave as they finish fill the SMs better than a
+// wave of blocks that stride: 2^24 options with one volatility 68 us against 71,
+// under the NT2 policy 137 against 152, and with a volatility table 141 against 162.
 constexpr int64_t kBsPipeMin = 1ll << 22;
 constexpr int kBsPipeStages = 3;
 
-template <class P, bool SIG_TAB, int STAGES>
-static nt2g_status launch_bs_pipe_n(const float *S, const float *K, const float *T, const float *sig, float sig_s,
-                                    float r, float *call, float *put, int64_t n, cudaStream_t st)
+static nt2g_status launch_bs_pipe(const float *S, const float *K, const float *T, const float *sig, float r, float *call,
+                                  float *put, int64_t n, cudaStream_t st)
 {
-    const size_t smem = (size_t)STAGES * (SIG_TAB ? 4 : 3) * 256 * sizeof(float4) + STAGES * sizeof(uint64_t);
-    static const cudaError_t attr = cudaFuncSetAttribute(k_bs_pipe<P, SIG_TAB, STAGES>,
-                                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const auto kernel = k_bs_pipe<kBsPipeStages>;
+    const size_t smem = (size_t)kBsPipeStages * 4 * 256 * sizeof(float4) + kBsPipeStages * sizeof(uint64_t);
+    static const cudaError_t attr = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (attr != cudaSuccess) return cuda_status(attr, "blackscholes pipeline: shared memory");
     int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_bs_pipe<P, SIG_TAB, STAGES>, 256, smem) !=
-            cudaSuccess || per_sm < 1)
-        per_sm = 1;
-    const int64_t tiles = n / 1024, full = (int64_t)device_sm_count() * per_sm;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 256, smem) != cudaSuccess || per_sm < 1) per_sm = 1;
+    const int64_t tiles = n / 1024, full = 2 * (int64_t)device_sm_count() * per_sm;
     const int grid = (int)(tiles < full ? tiles : full);
-    k_bs_pipe<P, SIG_TAB, STAGES><<<grid, 256, smem, st>>>(S, K, T, sig, sig_s, r, call, put, n);
+    kernel<<<grid, 256, smem, st>>>(S, K, T, sig, r, call, put, n);
     NT2G_LAUNCH_CHECK("blackscholes pipeline launch");
     return NT2G_OK;
 }
@@ -416,14 +411,8 @@ nt2g_status launch_bs(const float *S, const float *K, const float *T, const floa
         else k_bs<PP, TAB, false><<<grid_for(k_bs<PP, TAB, false>, n), 256, 0, st>>>(S, K, T, sig, sig_s, r,   \
                                                                                       call, put, n);           \
     } while (0)
-    if (vec && n >= kBsPipeMin) {
-        constexpr int ST = kBsPipeStages;
-        if (precision == NT2G_PREC_NT2)
-            return sig ? launch_bs_pipe_n<Nt2, true, ST>(S, K, T, sig, sig_s, r, call, put, n, st)
-                       : launch_bs_pipe_n<Nt2, false, ST>(S, K, T, sig, sig_s, r, call, put, n, st);
-        return sig ? launch_bs_pipe_n<Fast, true, ST>(S, K, T, sig, sig_s, r, call, put, n, st)
-                   : launch_bs_pipe_n<Fast, false, ST>(S, K, T, sig, sig_s, r, call, put, n, st);
-    }
+    if (vec && sig && precision != NT2G_PREC_NT2 && n >= kBsPipeMin)
+        return launch_bs_pipe(S, K, T, sig, r, call, put, n, st);
     if (precision == NT2G_PREC_NT2) {
         if (sig) NT2G_BS(Nt2, true);
         else NT2G_BS(Nt2, false);
