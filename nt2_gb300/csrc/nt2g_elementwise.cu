@@ -18,6 +18,19 @@ static int grid_for(KERN k, int64_t units)
     return persistent_blocks(k, kThreads, 0, kThreads * 2, units);
 }
 
+// `waves` waves of blocks at most, where SMs that finish first would wait for a
+// single wave's last blocks.  2^24 elements: rgb2yuv 67.8 us in one wave, 62.7 in
+// two, 60.1 in four, 58.8 with a thread a vector (2^20 pixels: 4.1, 3.8, 3.8, 3.8);
+// expr3 42.7, 41.9, 41.6, 44.1; saxpy, which does less a vector, 22.5, 22.7, 23.4,
+// 33.5 and stays with one.
+template <class KERN>
+static int grid_waves(KERN k, int64_t units, int waves)
+{
+    const int64_t one = grid_for(k, units), need = (units + kThreads - 1) / kThreads;
+    const int64_t g = one * waves;
+    return (int)(g < need ? g : need > 0 ? need : 1);
+}
+
 // ------------------------------------------------------------------ saxpy --
 // Y = alpha*X + Y with NT2's two roundings (demo/saxpy/nt2/saxpy_nt2.cpp:41).
 __global__ void __launch_bounds__(kThreads) k_saxpy(float alpha, const float *__restrict__ X,
@@ -90,9 +103,9 @@ nt2g_status launch_expr3(const float *x, const float *y, const float *z, float *
     if (n == 0) return NT2G_OK;
     int vec = aligned16(x) && aligned16(y) && aligned16(z) && aligned16(out);
     if (precision == NT2G_PREC_NT2)
-        k_expr3<Nt2><<<grid_for(k_expr3<Nt2>, (n + 3) / 4), kThreads, 0, st>>>(x, y, z, out, n, vec);
+        k_expr3<Nt2><<<grid_waves(k_expr3<Nt2>, (n + 3) / 4, 4), kThreads, 0, st>>>(x, y, z, out, n, vec);
     else
-        k_expr3<Fast><<<grid_for(k_expr3<Fast>, (n + 3) / 4), kThreads, 0, st>>>(x, y, z, out, n, vec);
+        k_expr3<Fast><<<grid_waves(k_expr3<Fast>, (n + 3) / 4, 4), kThreads, 0, st>>>(x, y, z, out, n, vec);
     NT2G_LAUNCH_CHECK("expr3 launch");
     return NT2G_OK;
 }
@@ -133,9 +146,9 @@ nt2g_status launch_rgb2yuv(const float *r, const float *g, const float *b, float
     if (n == 0) return NT2G_OK;
     int vec = aligned16(r) && aligned16(g) && aligned16(b) && aligned16(y) && aligned16(u) && aligned16(v);
     if (precision == NT2G_PREC_NT2)
-        k_rgb2yuv<Nt2><<<grid_for(k_rgb2yuv<Nt2>, (n + 3) / 4), kThreads, 0, st>>>(r, g, b, y, u, v, n, vec);
+        k_rgb2yuv<Nt2><<<grid_waves(k_rgb2yuv<Nt2>, (n + 3) / 4, 8), kThreads, 0, st>>>(r, g, b, y, u, v, n, vec);
     else
-        k_rgb2yuv<Fast><<<grid_for(k_rgb2yuv<Fast>, (n + 3) / 4), kThreads, 0, st>>>(r, g, b, y, u, v, n, vec);
+        k_rgb2yuv<Fast><<<grid_waves(k_rgb2yuv<Fast>, (n + 3) / 4, 8), kThreads, 0, st>>>(r, g, b, y, u, v, n, vec);
     NT2G_LAUNCH_CHECK("rgb2yuv launch");
     return NT2G_OK;
 }
