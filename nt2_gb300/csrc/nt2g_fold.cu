@@ -32,6 +32,7 @@ static_assert((int)SUM == (int)NT2G_FOLD_SUM &&
 
 constexpr int kFoldThreads = kThreads;
 constexpr int64_t kChunk = 16384;        // elements per chunk a contiguous fold asks workspace for
+constexpr int64_t kWave = 152 * 4;       // blocks the GPU holds at once
 constexpr int64_t kBlocks = 152 * 12;    // blocks a fold is cut into at least: a few waves, so that none is nearly empty
 constexpr int64_t kSmallSeg = 64;        // (many) segments up to this length: one thread each
 
@@ -174,7 +175,13 @@ static FoldPlan plan_fold(int64_t lo, int64_t inner, int64_t hi, bool aligned, i
         if (p.group == 1 && inner > 512 && hi < (inner <= 2048 ? 152 * 8 : 152 * 24)) p.group = 2;
         p.chunk = inner > 0 ? inner : 1;
         if (p.group == 2 && hi < kBlocks) {
-            const int64_t per = (kBlocks + hi - 1) / hi;
+            // one wave of four blocks an SM for a few long segments (2^24 elements:
+            // a sum of exponentials and a maximum 26.0 and 16.9 us in 1824 blocks,
+            // 22.3 and 13.2 in 608, 27.1 and 15.8 in 912; their partials 12.2 us to
+            // combine, now 7.3); more, and shorter, blocks for more segments and for
+            // tables far larger than the L2 cache, where the wave's last blocks cost
+            // more than that (10^8 elements: 120 and 118 us)
+            const int64_t per = hi <= kWave / 2 && inner * hi <= 1 << 25 ? kWave / hi : (kBlocks + hi - 1) / hi;
             int64_t chunk = (inner + per - 1) / per;
             if (chunk < 4096) chunk = 4096;
             p.chunk = (chunk + 1023) / 1024 * 1024;
