@@ -52,6 +52,7 @@
 #if !defined(__CUDACC_RTC__)
 #include <stdint.h>
 #include "nt2g_accum.cuh"
+#include "nt2g_f2.cuh"
 #define NT2G_FOLD_INF __builtin_huge_valf()
 #else
 #define NT2G_FOLD_INF __int_as_float(0x7f800000)
@@ -308,68 +309,37 @@ __device__ __forceinline__ void Total<OP>::put(float *out, int64_t *index, doubl
 // rounds as the scalar operation does), which halves the issue slots of its 28
 // operations an element pair.
 struct VarAcc {
-    typedef unsigned long long F2;
-    F2 s1, c1, s2, c2, p;
-    static __device__ __forceinline__ F2 pack(float a, float b)
-    {
-        F2 r;
-        asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-        return r;
-    }
-    static __device__ __forceinline__ float half(F2 v, int i)
+    f2 s1, c1, s2, c2, p;
+    static __device__ __forceinline__ float half(f2 v, int i)
     {
         float a, b;
-        asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+        upk(v, a, b);
         return i ? b : a;
     }
-    static __device__ __forceinline__ F2 add(F2 a, F2 b)
+    static __device__ __forceinline__ void csum2(f2 &s, f2 &c, f2 v)
     {
-        F2 r;
-        asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-        return r;
-    }
-    static __device__ __forceinline__ F2 sub(F2 a, F2 b)
-    {
-        F2 r;
-        asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-        return r;
-    }
-    static __device__ __forceinline__ F2 mul(F2 a, F2 b)
-    {
-        F2 r;
-        asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-        return r;
-    }
-    static __device__ __forceinline__ F2 fma(F2 a, F2 b, F2 c)
-    {
-        F2 r;
-        asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-        return r;
-    }
-    static __device__ __forceinline__ void csum2(F2 &s, F2 &c, F2 v)
-    {
-        const F2 t = add(s, v), bb = sub(t, s);
-        c = add(c, add(sub(s, sub(t, bb)), sub(v, bb)));
+        const f2 t = add2(s, v), bb = sub2(t, s);
+        c = add2(c, add2(sub2(s, sub2(t, bb)), sub2(v, bb)));
         s = t;
     }
     __device__ __forceinline__ void start(float pivot, float pivot1)
     {
-        s1 = c1 = s2 = c2 = pack(0.0f, 0.0f);
-        p = pack(pivot, pivot1);
+        s1 = c1 = s2 = c2 = dup(0.0f);
+        p = pk(pivot, pivot1);
     }
-    __device__ __forceinline__ void take2(F2 x)
+    __device__ __forceinline__ void take2(f2 x)
     {
-        const F2 d = sub(x, p), nd = sub(p, x);
-        const F2 bb = sub(d, x);  // TwoSum of x and -p: bb is -p's share
-        const F2 dl = sub(sub(x, sub(d, bb)), add(p, bb));
-        const F2 q = mul(d, d);
+        const f2 d = sub2(x, p), nd = negx2(d);
+        const f2 bb = sub2(d, x);  // TwoSum of x and -p: bb is -p's share
+        const f2 dl = sub2(sub2(x, sub2(d, bb)), add2(p, bb));
+        const f2 q = mul2(d, d);
         csum2(s1, c1, d);
-        c1 = add(c1, dl);
+        c1 = add2(c1, dl);
         csum2(s2, c2, q);
-        c2 = sub(c2, fma(add(nd, nd), dl, fma(nd, d, q)));  // less q - d^2 - 2 d dl
+        c2 = sub2(c2, fma2(add2(nd, nd), dl, fma2(nd, d, q)));  // less q - d^2 - 2 d dl
     }
     // one element: the other half adds zero
-    __device__ __forceinline__ void take(float x) { take2(pack(x, half(p, 1))); }
+    __device__ __forceinline__ void take(float x) { take2(pk(x, half(p, 1))); }
     __device__ __forceinline__ Sums sums() const
     {
         Sums r{CSum{half(s1, 0), half(c1, 0)}, CSum{half(s2, 0), half(c2, 0)}, half(p, 0)};
@@ -620,8 +590,8 @@ __device__ __forceinline__ void inner_body(const Src &src, int64_t inner, int64_
                 for (int u = 0; u < U; ++u) {
                     if (u >= n) break;
                     if constexpr (is_var(OP) && V == 4) {
-                        var.take2(VarAcc::pack(e[u][0], e[u][1]));
-                        var.take2(VarAcc::pack(e[u][2], e[u][3]));
+                        var.take2(pk(e[u][0], e[u][1]));
+                        var.take2(pk(e[u][2], e[u][3]));
                     } else {
 #pragma unroll
                         for (int v = 0; v < V; ++v) {
@@ -865,7 +835,7 @@ __device__ __forceinline__ void outer_body(const Src &src, int64_t lo, int64_t i
 #pragma unroll
                     for (int v = 0; v < VEC; ++v) {
                         if constexpr (is_var(OP)) {  // (VEC == 1: both halves the same)
-                            if (v % 2 == 0) var[v / 2].take2(VarAcc::pack(e[u][v], e[u][v + (VEC > 1)]));
+                            if (v % 2 == 0) var[v / 2].take2(pk(e[u][v], e[u][v + (VEC > 1)]));
                         } else if constexpr (OP == PROD) {
                             prod[v] *= (double)e[u][v];
                         } else {

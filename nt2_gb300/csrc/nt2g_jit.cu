@@ -840,12 +840,13 @@ std::vector<int> vjp_scalar_slots(const std::vector<nt2g_op> &ops, const std::ve
 constexpr size_t kVjpRing = 8;  // 2 x 8 x 256 x 8 bytes: 32 KB
 
 // The reverse-mode kernel of a program: each thread recomputes the forward
-// values of 4 consecutive elements (the statements of jit_source, so the
-// same bits as nt2g_eval), seeds the adjoints of the values stored into each
+// values of 2 consecutive elements (the statements of jit_source, so the
+// same bits as nt2g_eval; four need more registers than the loads they save), seeds the adjoints of the values stored into each
 // output slot with that slot's cotangent table, runs the adjoint rules in
 // reverse instruction order, and writes the adjoints of the loaded values to
 // the slots' gradient tables.  Adjoints of float scalars are summed per
-// thread in FP64, then per block (fixed order) into partials[block][scalar].
+// thread (vjp::ScalarSum), then per block in FP64 (fixed order) into
+// partials[block][scalar].
 std::string jit_vjp_source(const std::vector<nt2g_op> &ops, const std::vector<uint8_t> &logical, int precision,
                            std::string *why)
 {
@@ -904,7 +905,7 @@ std::string jit_vjp_source(const std::vector<nt2g_op> &ops, const std::vector<ui
         s += "}\n";
     }
     s += "template <class P, bool FULL>\n__device__ __forceinline__ void vjp_tile(const JitArgs &a, const VjpArgs &g, "
-         "const JitIn &in, long long i, int cnt, nt2g::CSum (&sacc)[NT2G_NS])\n{\n    typedef nt2g::Fast D;\n    constexpr int L = 2, A = 2;\n";
+         "const JitIn &in, long long i, int cnt, nt2g::vjp::ScalarSum (&sacc)[NT2G_NS])\n{\n    typedef nt2g::Fast D;\n    constexpr int L = 2, A = 2;\n";
     emit_body(s, ops, logical, false, true);
     for (size_t k = 0; k < ops.size(); ++k)
         if (act[k]) s += "    float g" + std::to_string(k) + "[A] = {0.0f, 0.0f};\n";
@@ -947,13 +948,13 @@ std::string jit_vjp_source(const std::vector<nt2g_op> &ops, const std::vector<ui
     for (int q = 0; q < ns; ++q)
         for (size_t k = 0; k < ops.size(); ++k)
             if (ops[k].code == NT2G_OP_SCALAR && act[k] && ops[k].a == sslots[q])
-                s += "    NT2G_LL if (j < cnt) nt2g::csum_add(sacc[" + std::to_string(q) + "], g" + std::to_string(k) + "[j]);\n";
+                s += "    sacc[" + std::to_string(q) + "].add(g" + std::to_string(k) + "[0], cnt > 1 ? g" + std::to_string(k) + "[1] : 0.0f);\n";
     s += "}\n\n";
     s += "extern \"C\" __global__ void __launch_bounds__(256) nt2g_vjp_kernel(const JitArgs a, const VjpArgs g, "
          "long long n, int vec, double *partials)\n{\n";
     s += precision == NT2G_PREC_NT2 ? "    typedef nt2g::Nt2 P;\n" : "    typedef nt2g::Fast P;\n";
-    s += "    nt2g::CSum sacc[NT2G_NS];\n"
-         "    for (int q = 0; q < NT2G_NS; ++q) sacc[q] = nt2g::CSum{0.0f, 0.0f};\n"
+    s += "    nt2g::vjp::ScalarSum sacc[NT2G_NS];\n"
+         "    for (int q = 0; q < NT2G_NS; ++q) sacc[q].start();\n"
          "    const long long stride = (long long)gridDim.x * blockDim.x * 2;\n"
          "    long long i = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * 2;\n";
     if (ring)
@@ -985,7 +986,7 @@ std::string jit_vjp_source(const std::vector<nt2g_op> &ops, const std::vector<ui
     if (ns > 0)
         s += "    __shared__ double red[8][NT2G_NS];\n"
              "    for (int q = 0; q < NT2G_NS; ++q) {\n"
-             "        double x = (double)sacc[q].s + (double)sacc[q].c;\n"
+             "        double x = sacc[q].total();\n"
              "        for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);\n"
              "        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5][q] = x;\n"
              "    }\n"

@@ -10,6 +10,38 @@
 namespace nt2g {
 namespace vjp {
 
+// A thread's share of a scalar's gradient: three floats a lane, each carrying the
+// rounding errors of the one before (72 bits, more than the FP64 sums of the
+// blocks that follow; an FP64 addition and its conversion here would hold a warp
+// for 32 cycles an element).  Adjoints that could overflow them, infinities and
+// NaN go to FP64 at once.
+struct ScalarSum {
+    f2 s, c, d;
+    double far;
+    __device__ __forceinline__ void start() { s = c = d = dup(0.0f); far = 0.0; }
+    __device__ __forceinline__ void add(float g0, float g1)
+    {
+        if (!(fabsf(g0) < 0x1p96f && fabsf(g1) < 0x1p96f)) {
+            far += (double)g0 + (double)g1;
+            return;
+        }
+        const f2 g = pk(g0, g1), t = add2(s, g), b = sub2(t, s), e = add2(sub2(s, sub2(t, b)), sub2(g, b));
+        const f2 u = add2(c, e), v = sub2(u, c);
+        d = add2(d, add2(sub2(c, sub2(u, v)), sub2(e, v)));
+        s = t;
+        c = u;
+    }
+    __device__ __forceinline__ double total() const
+    {
+        float s0, s1, c0, c1, d0, d1;
+        upk(s, s0, s1);
+        upk(c, c0, c1);
+        upk(d, d0, d1);
+        return far + (((double)d0 + (double)d1) + ((double)c0 + (double)c1) + ((double)s0 + (double)s1));
+    }
+};
+
+
 constexpr float kPi = 3.14159265358979323846f;
 constexpr float kLn2 = 0.693147180559945309417f;
 constexpr float kLn10 = 2.30258509299404568402f;

@@ -55,3 +55,25 @@ def test_reverse_mode_ahead_matches_element_by_element(lib, dev, n, form):
             assert torch.equal(u.view(torch.int32), v.view(torch.int32))
         # every addend within 2^-46 of its sum's magnitude: log, exp and the cotangents stay below 100
         assert abs(float(a[-1]) - float(b[-1])) <= 2.0 ** -44 * n * 100.0
+
+
+@pytest.mark.parametrize("n", [1, 2, 513, 300_001])
+def test_scalar_gradient_of_extreme_adjoints(lib, dev, n):
+    """A scalar's gradient in FP64 range: adjoints past 2^96 whose float sum would
+    overflow, huge ones that cancel, infinities and NaN."""
+    x = np.full(n, 1.0, np.float32)
+    for big in (np.float32(3e38), np.float32(2.0 ** 96), np.float32(-1e30)):
+        t, ct = torch.from_numpy(x).to(dev), torch.full((n,), float(big), device=dev)
+        if n > 2:
+            ct[1::2] = -float(big)
+            ct[0] = 1.0
+        r = E.Scalar(0.5)
+        (g,) = E.vjp([torch.empty_like(t)], [E.Table(t) * r], [ct], [r])
+        want = ct.double().sum().item()
+        assert abs(float(g) - want) <= 2.0 ** -50 * float(ct.double().abs().sum())
+    ct = torch.ones(n, device=dev)
+    for v in (float("inf"), float("-inf"), float("nan")):
+        ct[n // 2] = v
+        r = E.Scalar(0.5)
+        (g,) = E.vjp([torch.empty_like(t)], [E.Table(t) * r], [ct], [r])
+        assert (np.isnan(float(g)) if np.isnan(v) else float(g) == v)
