@@ -34,13 +34,21 @@ inline bool aligned16(const void *p) { return ((uintptr_t)p & 15u) == 0; }
 // reads only inputs no earlier kernel writes before pdl_wait(), and writes
 // nothing before it.  pdl_trigger() lets the next dependent launch begin.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// The same for a kernel that reads its tables through pointers the compiler takes
+// for read-only: they count as new from here on, so no load moves ahead of the wait.
+template <class P> __device__ __forceinline__ void pdl_new(P &p) { asm volatile("" : "+l"(p)::"memory"); }
+template <class... P> __device__ __forceinline__ void pdl_wait_for(P &...p)
+{
+    pdl_wait();
+    (pdl_new(p), ...);
+}
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 template <class... KArgs, class... Args>
-inline cudaError_t launch_dependent(void (*kernel)(KArgs...), int grid, int block, cudaStream_t st, Args... args)
+inline cudaError_t launch_dependent(void (*kernel)(KArgs...), dim3 grid, int block, cudaStream_t st, Args... args)
 {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
+    cfg.gridDim = grid;
     cfg.blockDim = dim3(block);
     cfg.dynamicSmemBytes = 0;
     cfg.stream = st;
