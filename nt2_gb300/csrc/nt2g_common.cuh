@@ -32,7 +32,10 @@ inline bool aligned16(const void *p) { return ((uintptr_t)p & 15u) == 0; }
 // still running; pdl_wait() returns once that kernel has completed and its
 // memory is visible (immediately when there is no such dependency).  A kernel
 // reads only inputs no earlier kernel writes before pdl_wait(), and writes
-// nothing before it.  pdl_trigger() lets the next dependent launch begin.
+// nothing before it.  pdl_trigger() lets the next dependent launch begin; at a
+// kernel's start, it lets the next kernel's blocks line up once all of this one's
+// run.  (Folds, their combining kernels and the median's passes: 9 and 8 launches
+// of a table's six statistics and three medians, 286 -> 266 and 142 -> 128 us.)
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // The same for a kernel that reads its tables through pointers the compiler takes
 // for read-only: they count as new from here on, so no load moves ahead of the wait.

@@ -58,6 +58,8 @@ __global__ void __launch_bounds__(kFoldThreads, is_var(OP) ? 3 : 4) k_fold_inner
                                                              float *__restrict__ out, int64_t *__restrict__ index,
                                                              const float *__restrict__ cen, double *__restrict__ out64)
 {
+    pdl_trigger();  // the kernel that combines the partials lines up
+    pdl_wait_for(src.x, part, out, index, cen, out64);
     inner_body<RawSrc, OP, FINAL, IDX, G>(src, inner, hi, chunk, q, vec, part, out, index, cen, out64);
 }
 
@@ -75,6 +77,8 @@ __global__ void __launch_bounds__(kFoldThreads, is_var(OP) ? 3 : 4) k_fold_outer
                                                              float *__restrict__ out, int64_t *__restrict__ index,
                                                              const float *__restrict__ cen, double *__restrict__ out64)
 {
+    pdl_trigger();
+    pdl_wait_for(src.x, part, out, index, cen, out64);
     outer_body<RawSrc, OP, VEC, FINAL>(src, lo, inner, hi, ck, q, part, out, index, cen, out64);
 }
 
@@ -97,6 +101,8 @@ __global__ void __launch_bounds__(kFoldThreads) k_fold_finish(const Partial *__r
                                                               const float *__restrict__ cen, double *__restrict__ out64)
 {
     __shared__ Total<OP> st[kRanges][32];
+    pdl_trigger();
+    pdl_wait_for(part, out, index, cen, out64);
     const int lane = threadIdx.x & 31, range = threadIdx.x >> 5;
     const int64_t per = (q + kRanges - 1) / kRanges, c0 = range * per, c1 = c0 + per < q ? c0 + per : q;
     for (int64_t o0 = (int64_t)blockIdx.x * 32; o0 < n_out; o0 += (int64_t)gridDim.x * 32) {
@@ -131,6 +137,8 @@ __global__ void __launch_bounds__(kFoldThreads) k_fold_finish_block(const Partia
                                                                     double *__restrict__ out64)
 {
     __shared__ Total<OP> st[kFoldThreads];
+    pdl_trigger();
+    pdl_wait_for(part, out, index, cen, out64);
     const int64_t per = (q + kFoldThreads - 1) / kFoldThreads, c0 = threadIdx.x * per,
                   c1 = c0 + per < q ? c0 + per : q;
     for (int64_t o = blockIdx.x; o < n_out; o += gridDim.x) {
@@ -358,8 +366,8 @@ static nt2g_status launch_fold_op(const FoldInput &in, int64_t lo, int64_t inner
         int64_t chunk = p.chunk, q = p.q;
         int vec = p.vec;
         if (!in.expr) {
-#define NT2G_INNER(F, I, G) k_fold_inner<OP, F, I, G><<<g, kFoldThreads, 0, st>>>(src, inner, hi, chunk, q, vec, part, out, \
-                                                                               index, cen, out64)
+#define NT2G_INNER(F, I, G) ce = launch_dependent(k_fold_inner<OP, F, I, G>, g, kFoldThreads, st, src, inner, hi, chunk, q, vec,  \
+                                                  part, out, index, cen, out64)
 #define NT2G_INNER_I(F, G) do { if (EXT && idx) NT2G_INNER(F, EXT, G); else NT2G_INNER(F, false, G); } while (0)
             constexpr bool EXT = OP == MAX || OP == MIN;  // only these have positions
             if (!fin) NT2G_INNER_I(false, 256);
@@ -368,7 +376,6 @@ static nt2g_status launch_fold_op(const FoldInput &in, int64_t lo, int64_t inner
             else NT2G_INNER_I(true, 256);
 #undef NT2G_INNER_I
 #undef NT2G_INNER
-            ce = cudaGetLastError();
         } else {
             void *pr[] = {(void *)jargs, &inner, &hi, &chunk, &q, &vec, &part, &out, &index, &cen, &out64};
             ce = launch_by_handle(jk->inner[fin ? p.group : 3][idx], g, pr, st);
@@ -379,12 +386,11 @@ static nt2g_status launch_fold_op(const FoldInput &in, int64_t lo, int64_t inner
         const bool fin = p.q == 1;
         int64_t chunk = p.chunk, q = p.q;
         if (!in.expr) {
-#define NT2G_OUTER(V, F) k_fold_outer<OP, V, F><<<g, kFoldThreads, 0, st>>>(src, lo, inner, hi, chunk, q, part, out, \
-                                                                            index, cen, out64)
+#define NT2G_OUTER(V, F) ce = launch_dependent(k_fold_outer<OP, V, F>, g, kFoldThreads, st, src, lo, inner, hi, chunk, q, part, out, \
+                                               index, cen, out64)
             if (p.vec == 4) { if (fin) NT2G_OUTER(4, true); else NT2G_OUTER(4, false); }
             else { if (fin) NT2G_OUTER(1, true); else NT2G_OUTER(1, false); }
 #undef NT2G_OUTER
-            ce = cudaGetLastError();
         } else {
             void *pr[] = {(void *)jargs, &lo, &inner, &hi, &chunk, &q, &part, &out, &index, &cen, &out64};
             ce = launch_by_handle(jk->outer[p.vec == 4][fin], g, pr, st);
@@ -394,11 +400,12 @@ static nt2g_status launch_fold_op(const FoldInput &in, int64_t lo, int64_t inner
     if (p.q > 1 && p.kind != 0) {
         // a block per output where eight threads each would walk long ranges
         if (n_out < 32 || (n_out <= 2048 && p.q > 128))
-            k_fold_finish_block<OP><<<cap(n_out), kFoldThreads, 0, st>>>(part, n_out, p.q, p.chunk, inner, out, index, cen,
-                                                                        out64);
+            ce = launch_dependent(k_fold_finish_block<OP>, dim3(cap(n_out)), kFoldThreads, st, part, n_out, p.q, p.chunk, inner, out,
+                                  index, cen, out64);
         else
-            k_fold_finish<OP><<<cap((n_out + 31) / 32), kFoldThreads, 0, st>>>(
-                part, n_out, p.q, p.chunk, inner, out, index, cen, out64);
+            ce = launch_dependent(k_fold_finish<OP>, dim3(cap((n_out + 31) / 32)), kFoldThreads, st, part, n_out, p.q, p.chunk,
+                                  inner, out, index, cen, out64);
+        if (ce != cudaSuccess) return cuda_status(ce, "fold combine launch");
         NT2G_LAUNCH_CHECK("fold combine launch");
     }
     return NT2G_OK;

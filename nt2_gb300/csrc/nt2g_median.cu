@@ -277,6 +277,8 @@ __global__ void __launch_bounds__(MAXT, MAXT < 1024 ? 1536 / MAXT : 1) k_median_
     __shared__ uint32_t list[S][kList];
     __shared__ uint32_t s_prefix[S], s_r[S], s_cnt[S], s_m[S], s_up[S];
     __shared__ int s_bits[S], s_nan[S];
+    pdl_trigger();
+    pdl_wait_for(x, centre, out);
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, slot = tid % S;
     const int per = blockDim.x / S;  // threads a slice
     const int64_t groups = (lo + S - 1) / S, h = blockIdx.x / groups, l0 = (blockIdx.x - h * groups) * S;
@@ -386,6 +388,8 @@ constexpr uint32_t kDone = 0x80000000u;  // in nan: the slice's result is writte
 
 __global__ void k_median_init(MedState *st, unsigned long long *ghist, int64_t S, int64_t n)
 {
+    pdl_trigger();
+    pdl_wait_for(st, ghist);
     const int64_t s = blockIdx.x;
     for (int i = threadIdx.x; i < 256; i += blockDim.x) ghist[s * 256 + i] = 0;
     if (threadIdx.x == 0) st[s] = MedState{(unsigned long long)((n - 1) >> 1), (unsigned long long)n, 0, 0, 0xffffffffu, 0};
@@ -409,6 +413,8 @@ __global__ void __launch_bounds__(256, 6) k_median_pass(const float *__restrict_
     __shared__ uint32_t hist[256];
     __shared__ uint32_t list[kList];
     __shared__ uint32_t s_last;
+    pdl_trigger();  // the next pass lines up while this one runs
+    pdl_wait_for(x, centre, st, ghist, out);
     const int64_t s = s0 + blockIdx.y, l = s % lo, h = s / lo;
     MedState *ms = st + s;
     unsigned long long *gh = ghist + s * 256;
@@ -524,7 +530,7 @@ size_t median_workspace_bytes(int64_t lo, int64_t n, int64_t hi)
 // The fewest keys a thread whose block stays within 1024 threads: more threads
 // a slice hide more of its phases.
 template <bool AD, int S>
-static void launch_regs(const float *x, int64_t lo, int64_t n, int64_t hi, const float *centre, float *out, cudaStream_t st)
+static cudaError_t launch_regs(const float *x, int64_t lo, int64_t n, int64_t hi, const float *centre, float *out, cudaStream_t st)
 {
     const unsigned grid = (unsigned)((lo + S - 1) / S * hi);
     const int64_t keys = n * S;
@@ -532,7 +538,7 @@ static void launch_regs(const float *x, int64_t lo, int64_t n, int64_t hi, const
         const int64_t per = (n + kpt - 1) / kpt;
         return (int)((per * S + 31) / 32 * 32);
     };
-#define NT2G_REGS(KPT, MAXT) k_median_regs<AD, S, KPT, MAXT><<<grid, threads(KPT), 0, st>>>(x, lo, n, centre, out)
+#define NT2G_REGS(KPT, MAXT) return launch_dependent(k_median_regs<AD, S, KPT, MAXT>, dim3(grid), threads(KPT), st, x, lo, n, centre, out)
     if (keys <= 16 * 256) NT2G_REGS(16, 256);
     else if (keys <= 16 * 768) NT2G_REGS(16, 768);
     else if (keys <= 16 * 1024) NT2G_REGS(16, 1024);
@@ -554,15 +560,17 @@ static nt2g_status median_pass(const float *x, int64_t lo, int64_t n, int64_t hi
         return NT2G_OK;
     }
     if (n <= kRegKeys) {
-        if (lo >= 8 && n * 8 <= kRegKeys) launch_regs<AD, 8>(x, lo, n, hi, centre, out, st);
-        else if (lo >= 4 && n * 4 <= kRegKeys) launch_regs<AD, 4>(x, lo, n, hi, centre, out, st);
-        else launch_regs<AD, 1>(x, lo, n, hi, centre, out, st);
+        cudaError_t ce;
+        if (lo >= 8 && n * 8 <= kRegKeys) ce = launch_regs<AD, 8>(x, lo, n, hi, centre, out, st);
+        else if (lo >= 4 && n * 4 <= kRegKeys) ce = launch_regs<AD, 4>(x, lo, n, hi, centre, out, st);
+        else ce = launch_regs<AD, 1>(x, lo, n, hi, centre, out, st);
+        if (ce != cudaSuccess) return cuda_status(ce, "median (registers)");
         NT2G_LAUNCH_CHECK("median (registers)");
         return NT2G_OK;
     }
     unsigned long long *ghist = (unsigned long long *)ws;
     MedState *state = (MedState *)(ghist + S * 256);
-    k_median_init<<<(unsigned)S, 256, 0, st>>>(state, ghist, S, n);
+    cudaError_t ce = launch_dependent(k_median_init, dim3((unsigned)S), 256, st, state, ghist, S, n);
     // one wave of blocks (six an SM), of at least 4096 elements each
     int64_t chunk = (n * S + 152 * 6 - 1) / (152 * 6);
     chunk = chunk < 4096 ? 4096 : chunk > 65536 ? 65536 : (chunk + 255) / 256 * 256;
@@ -570,12 +578,12 @@ static nt2g_status median_pass(const float *x, int64_t lo, int64_t n, int64_t hi
     for (int above = 32; above >= 0; above -= 8) {
         for (int64_t s0 = 0; s0 < S; s0 += 65535) {  // grid.y: at most 65535 slices per launch
             const dim3 grid(chunks, (unsigned)(S - s0 < 65535 ? S - s0 : 65535));
-            if (lo == 1)
-                k_median_pass<AD, true><<<grid, 256, 0, st>>>(x, lo, n, chunk, centre, state, ghist, above, s0, out);
-            else
-                k_median_pass<AD, false><<<grid, 256, 0, st>>>(x, lo, n, chunk, centre, state, ghist, above, s0, out);
+            if (ce != cudaSuccess) return cuda_status(ce, "median (global passes)");
+            ce = launch_dependent(lo == 1 ? k_median_pass<AD, true> : k_median_pass<AD, false>, grid, 256, st, x, lo, n, chunk, centre,
+                                  state, ghist, above, s0, out);
         }
     }
+    if (ce != cudaSuccess) return cuda_status(ce, "median (global passes)");
     NT2G_LAUNCH_CHECK("median (global passes)");
     return NT2G_OK;
 }

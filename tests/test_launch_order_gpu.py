@@ -83,3 +83,39 @@ def test_chained_calls_in_a_graph_of_two_streams(lib, dev):
         torch.cuda.synchronize()
         for b, w in zip(bufs, want):
             assert torch.equal(b.view(torch.int32), w.view(torch.int32))
+
+
+def _folds_chain(lib, step, rows, cols, dev):
+    g = torch.Generator(device=dev)
+    g.manual_seed(rows)
+    t = torch.rand(rows * cols, device=dev, generator=g) * 4 + 1
+    seen = []
+    for k in range(3):
+        for op in ("mean", "stdev", "max"):
+            down = lib.fold(t, 1, rows, cols, op)        # along columns
+            step()
+            across = lib.fold(t, rows, cols, 1, op)      # along rows
+            step()
+            both = lib.fold(down, 1, cols, 1, op)        # of what was just written
+            step()
+            t[:cols] = down                              # feed the next calls
+            t[-rows:] = across
+            t[0] += both[0]
+            step()
+            seen += [down, across, both]
+        for shape in ((1, rows, cols), (rows, cols, 1), (1, rows * cols, 1)):
+            m = lib.median(t, *shape)
+            step()
+            t[k:k + m.numel()] += m * 0.25
+            step()
+            seen.append(m)
+    return [s.clone() for s in seen + [t]]
+
+
+@pytest.mark.parametrize("rows,cols", [(40, 60), (3000, 17), (1500, 1100), (300, 3001), (50000, 4)])
+def test_chained_folds_and_medians(lib, dev, rows, cols):
+    want = _folds_chain(lib, torch.cuda.synchronize, rows, cols, dev)
+    got = _folds_chain(lib, lambda: None, rows, cols, dev)
+    torch.cuda.synchronize()
+    for w, x in zip(want, got):
+        assert torch.equal(w.view(torch.int32), x.view(torch.int32))
