@@ -834,8 +834,8 @@ std::vector<int> vjp_scalar_slots(const std::vector<nt2g_op> &ops, const std::ve
 
 // A thread's next elements wait in its own slots of shared memory (one pair of
 // each table ahead), so their loads run beside the arithmetic without holding
-// registers (2^24 options' reverse mode: 174 us, stalled on loads in half of
-// its cycles, without; 167 with); programs of more than kVjpRing tables load
+// registers (2^24 options' reverse mode, scalar sums in two floats: 174 us,
+// stalled on loads in half of its cycles, without; 167 with); programs of more than kVjpRing tables load
 // directly.
 constexpr size_t kVjpRing = 8;  // 2 x 8 x 256 x 8 bytes: 32 KB
 

@@ -13,7 +13,8 @@ namespace vjp {
 // A thread's share of a scalar's gradient: three floats a lane, each carrying the
 // rounding errors of the one before (72 bits, more than the FP64 sums of the
 // blocks that follow; an FP64 addition and its conversion here would hold a warp
-// for 32 cycles an element).  Adjoints that could overflow them, infinities and
+// for 32 cycles an element; two floats lost the last bits: 162 us for 2^24
+// options with them, 171 with three).  Adjoints that could overflow them, infinities and
 // NaN go to FP64 at once.
 struct ScalarSum {
     f2 s, c, d;
