@@ -413,6 +413,20 @@ template <bool MX, bool FIRST, int W> struct BatchRun {
                         if (u < n && e[u][c] == m) ifirst = pos + u * step + c;
                 ilast = ifirst;
             }
+        } else if (m == (MX ? -NT2G_FOLD_INF : NT2G_FOLD_INF)) {
+            // nothing but the neutral value so far (masked elements, logarithms of
+            // zeros): it is no better than itself, yet its first position counts
+            v = m;
+            if (U * V == 1 || ifirst < 0) {
+#pragma unroll
+                for (int u = U - 1; u >= 0; --u)
+#pragma unroll
+                    for (int c = V - 1; c >= 0; --c) {
+                        const int32_t at = pos + u * step + c;
+                        if (u < n && e[u][c] == m && (unsigned)at < (unsigned)ifirst) ifirst = at;
+                    }
+                ilast = ifirst;
+            }
         } else if (U * V == 1 && n && e[0][0] == m && m != 0.0f) {  // the ends of a segment come last
             ifirst = (unsigned)pos < (unsigned)ifirst ? pos : ifirst;
             ilast = ifirst;
