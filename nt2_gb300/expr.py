@@ -825,7 +825,7 @@ def _slot_of(slots, x):
         for i, s in enumerate(slots):
             if s is x:
                 return i
-    else:
+    elif isinstance(x, lib._pytorch().Tensor):
         at, dtype = x.data_ptr(), x.dtype
         for i, s in enumerate(slots):
             if not isinstance(s, Node) and s.data_ptr() == at and s.dtype == dtype:
