@@ -35,6 +35,7 @@ constexpr int64_t kChunk = 16384;        // elements per chunk a contiguous fold
 constexpr int64_t kWave = 152 * 4;       // blocks the GPU holds at once
 constexpr int64_t kBlocks = 152 * 12;    // blocks a fold is cut into at least: a few waves, so that none is nearly empty
 constexpr int64_t kSmallSeg = 64;        // (many) segments up to this length: one thread each
+constexpr int64_t kMostPerThread = 512;  // elements of a contiguous segment that one thread sums
 
 // A table as a fold source: streaming loads.
 struct RawSrc {
@@ -177,12 +178,14 @@ static FoldPlan plan_fold(int64_t lo, int64_t inner, int64_t hi, bool aligned, i
         p.kind = 1;
         p.vec = aligned;
         // at least 32 elements (eight float4 loads) a thread, with more threads a
-        // segment where there are too few segments to fill the GPU
+        // segment where there are too few segments to fill the GPU, and at most 512:
+        // a thread's sum is a pair of floats, what it hands on FP64 within a warp
         p.group = inner <= 256 ? 0 : 1;
         if (p.group == 0 && inner > 64 && hi < 152 * 32) p.group = 1;
         if (p.group == 1 && inner > 512 && hi < (inner <= 2048 ? 152 * 8 : 152 * 24)) p.group = 2;
+        if (inner > kMostPerThread * 32) p.group = 2;
         p.chunk = inner > 0 ? inner : 1;
-        if (p.group == 2 && hi < kBlocks) {
+        if (p.group == 2 && (hi < kBlocks || inner > kMostPerThread * kFoldThreads)) {
             // one wave of four blocks an SM for a few long segments (2^24 elements:
             // a sum of exponentials and a maximum 26.0 and 16.9 us in 1824 blocks,
             // 22.3 and 13.2 in 608, 27.1 and 15.8 in 912; their partials 12.2 us to
@@ -192,6 +195,7 @@ static FoldPlan plan_fold(int64_t lo, int64_t inner, int64_t hi, bool aligned, i
             const int64_t per = hi <= kWave / 2 && inner * hi <= 1 << 25 ? kWave / hi : (kBlocks + hi - 1) / hi;
             int64_t chunk = (inner + per - 1) / per;
             if (chunk < 4096) chunk = 4096;
+            if (chunk > kMostPerThread * kFoldThreads) chunk = kMostPerThread * kFoldThreads;
             p.chunk = (chunk + 1023) / 1024 * 1024;
             p.q = (inner + p.chunk - 1) / p.chunk;
             if (p.q < 1) p.q = 1;

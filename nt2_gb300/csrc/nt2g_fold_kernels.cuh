@@ -37,11 +37,11 @@
 // pass, then the centred sum of squares.
 //
 // Fast policy: sums are compensated FP32 (TwoSum; squares carry their FMA
-// product error) per thread, chunks combined in FP64; var/stdev take one pass:
-// the deviations from an element of the chunk, and their squares, are summed
-// compensated, and chunks combine by their means in FP64 (a pivot among the
-// data keeps the correction to the mean at most n times the result); meanad
-// centres on the mean of a first pass; prod in FP64; max/min are exact.
+// product error) per thread and over a warp's lanes, warps and chunks combined
+// with the bits and the range of FP64; var/stdev take one pass: the deviations
+// from the mean of the chunk's first few elements, and their squares, are summed
+// compensated, and again about the chunk's own mean where that is far away;
+// meanad centres on the mean of a first pass; prod in FP64; max/min are exact.
 // Contiguous segments are folded by 8, 32 or 256 threads each (inner_body),
 // strided ones by warps over 32 columns (four each with 128-bit loads), rows
 // split over a block's warps (outer_body), so that a block hands on one
@@ -54,8 +54,10 @@
 #include "nt2g_accum.cuh"
 #include "nt2g_f2.cuh"
 #define NT2G_FOLD_INF __builtin_huge_valf()
+#define NT2G_FOLD_NAN __builtin_nanf("")
 #else
 #define NT2G_FOLD_INF __int_as_float(0x7f800000)
+#define NT2G_FOLD_NAN __int_as_float(0x7fffffff)
 #endif
 
 namespace nt2g {
@@ -182,21 +184,57 @@ template <int OP> __device__ __forceinline__ void sum_elem_c(CSum &a, float x, f
 }
 
 // ---------------------------------------------------------------- partials --
-// Per (chunk, output), chunk-major: a compensated sum (sums; variances: of the
-// deviations from the chunk's pivot, and of their squares), a product or a
-// Best.  Turned into FP64 only where many outputs or chunks are at hand at
-// once: an FP64 instruction takes a warp sixteen cycles, however few of its
-// lanes need it.
+// What a thread or a warp hands on: a compensated sum (variances: of the
+// deviations from the pivot, and of their squares), times `up`, which is one but
+// where lanes within the float range are not together (lanes_sums); a product; a
+// Best.
 struct Sums {
     CSum s1, s2;
-    float piv;
+    float piv, up;
 };
-struct Partial {
+struct Share {
     union {
         Sums v;
         double d;
         Best b;
     };
+};
+__device__ __forceinline__ double wide(const CSum &a, float up = 1.0f)
+{
+    const double t = (double)a.s + (double)a.c;
+    return up == 1.0f ? t : t * (double)up;
+}
+// What a block hands on per (chunk, output), chunk-major: its warps together, in
+// FP64.
+struct Partial {
+    union {
+        struct { double s1, s2; float piv; } v;
+        double d;
+        Best b;
+    };
+};
+
+// Three floats, each carrying the rounding errors of the one before: 72 bits, so
+// a block's warps combine with no fewer than FP64 has.  (An FP64 instruction
+// takes a warp sixteen cycles, however few of its lanes need it; the eight warps
+// of 128 outputs in FP64 would take 28 of them where this takes five.)
+struct Sum3 {
+    float s, c, d = 0.0f;
+    __device__ __forceinline__ explicit Sum3(const CSum &x) : s(x.s), c(x.c) {}
+    static __device__ __forceinline__ float two_sum(float &a, float b)
+    {
+        const float t = __fadd_rn(a, b), bb = __fsub_rn(t, a);
+        const float e = __fadd_rn(__fsub_rn(a, __fsub_rn(t, bb)), __fsub_rn(b, bb));
+        a = t;
+        return e;
+    }
+    __device__ __forceinline__ void add(const CSum &x)
+    {
+        const float e1 = two_sum(s, x.s), e2 = two_sum(c, x.c), e3 = two_sum(c, e1);
+        d = __fadd_rn(d, __fadd_rn(e2, e3));
+    }
+    __device__ __forceinline__ bool in_range() const { return s - s == 0.0f; }
+    __device__ __forceinline__ double wide() const { return (double)s + ((double)c + (double)d); }
 };
 
 // Chunks of one output combined in order.  A variance's sums are shifted to
@@ -209,19 +247,30 @@ template <int OP> struct Total {
     __device__ __forceinline__ void add(const Partial &p, double n)
     {
         if constexpr (is_var(OP)) {
-            const double s1 = (double)p.v.s1.s + (double)p.v.s1.c, s2 = (double)p.v.s2.s + (double)p.v.s2.c;
             if (!any) p0 = (double)p.v.piv;
             const double d = (double)p.v.piv - p0, nd = n * d;
-            t += s1 + nd;
-            t2 += s2 + d * (2.0 * s1 + nd);
+            t += p.v.s1 + nd;
+            t2 += p.v.s2 + d * (2.0 * p.v.s1 + nd);
             any = true;
         } else if constexpr (is_sum(OP)) {
-            t += (double)p.v.s1.s + (double)p.v.s1.c;
+            t += p.v.s1;
         } else if constexpr (OP == PROD) {
             t *= p.d;
         } else {
             b = best_merge<OP == MAX>(b, p.b);
         }
+    }
+    __device__ __forceinline__ void add(const Share &r, double n)
+    {
+        Partial p;
+        if constexpr (is_sum(OP)) p.v.s1 = wide(r.v.s1, r.v.up);
+        if constexpr (is_var(OP)) {
+            p.v.s2 = wide(r.v.s2, r.v.up);
+            p.v.piv = r.v.piv;
+        }
+        if constexpr (OP == PROD) p.d = r.d;
+        if constexpr (!is_sum(OP) && OP != PROD) p.b = r.b;
+        add(p, n);
     }
     __device__ __forceinline__ void add(const Total &o, double n)  // n: the elements of o
     {
@@ -342,21 +391,41 @@ struct VarAcc {
     __device__ __forceinline__ void take(float x) { take2(pk(x, half(p, 1))); }
     __device__ __forceinline__ Sums sums() const
     {
-        Sums r{CSum{half(s1, 0), half(c1, 0)}, CSum{half(s2, 0), half(c2, 0)}, half(p, 0)};
+        Sums r{CSum{half(s1, 0), half(c1, 0)}, CSum{half(s2, 0), half(c2, 0)}, half(p, 0), 1.0f};
         csum_merge(r.s1, CSum{half(s1, 1), half(c1, 1)});
         csum_merge(r.s2, CSum{half(s2, 1), half(c2, 1)});
         return r;
     }
-    // Squares past the float range though no element is infinite or not a
-    // number: the pivot may be far off, the mean is worth a second try.
-    static __device__ __forceinline__ bool over(const Sums &r)
+    // of one half alone
+    __device__ __forceinline__ Sums sums(int i, float piv) const
+    {
+        return Sums{CSum{half(s1, i), half(c1, i)}, CSum{half(s2, i), half(c2, i)}, piv, 1.0f};
+    }
+    // Whether the n deviations, summing to a and their squares to b, are worth
+    // summing again about their mean: squares past the float range though no
+    // element is infinite or not a number, or a pivot so far off (more than 2.8
+    // times the deviation; a trend's start is 1.7) that bringing the squares to the
+    // mean cancels more than three of their bits.
+    static __device__ __forceinline__ bool off(float a, float b, float n)
+    {
+        if (!(b - b == 0.0f)) return a - a == 0.0f;
+        return 1.125f * a * __fdividef(a, n) > b;
+    }
+    static __device__ __forceinline__ bool off(const Sums &r, int64_t n)
     {
         const float a = r.s1.s + r.s1.c, b = r.s2.s + r.s2.c;
-        return a - a == 0.0f && b - b != 0.0f;
+        return off(r.up == 1.0f ? a : a * 0x1p32f, b, (float)n);  // (squares scaled by 2^-64)
+    }
+    // of FP64 sums that may be out of the float range
+    static __device__ __forceinline__ bool off(double a, double b, int64_t n)
+    {
+        const float fb = (float)b;
+        if (fb - fb == 0.0f) return off((float)a, fb, (float)n);
+        return b - b == 0.0 ? 1.125 * a * (a / (double)n) > b : a - a == 0.0;
     }
     static __device__ __forceinline__ float mean(const Sums &r, int64_t n)
     {
-        return r.piv + (r.s1.s + r.s1.c) / (float)n;
+        return r.piv + r.up * __fdividef(r.s1.s + r.s1.c, (float)n);
     }
 };
 
@@ -378,7 +447,9 @@ __device__ __forceinline__ float min_nan(float a, float b)
     return r;
 }
 template <bool MX, bool FIRST, int W> struct BatchRun {
-    float cur = MX ? -NT2G_FOLD_INF : NT2G_FOLD_INF, v = 0.0f;
+    // not a number: nothing yet, so the first batch's extreme is a new one whatever
+    // it is, the neutral infinity too (masked elements, logarithms of zeros)
+    float cur = NT2G_FOLD_NAN, v = 0.0f;
     int32_t ifirst = -1, ilast = -1, inan = -1;
     // elements e[u][c], u < n, at positions pos + u * step + c
     template <int U, int V>
@@ -400,7 +471,7 @@ template <bool MX, bool FIRST, int W> struct BatchRun {
         if (better<MX>(cur, m)) return;
         // Equal numbers have equal bits but for zeros, so only there does the last
         // one matter; otherwise the first position of a new extreme is all.
-        if (better<MX>(m, cur)) {
+        if (m == m && m != cur) {
             cur = v = m;
             ifirst = ilast = -1;
             if (!FIRST && m != 0.0f) {
@@ -411,20 +482,6 @@ template <bool MX, bool FIRST, int W> struct BatchRun {
 #pragma unroll
                     for (int c = V - 1; c >= 0; --c)
                         if (u < n && e[u][c] == m) ifirst = pos + u * step + c;
-                ilast = ifirst;
-            }
-        } else if (m == (MX ? -NT2G_FOLD_INF : NT2G_FOLD_INF)) {
-            // nothing but the neutral value so far (masked elements, logarithms of
-            // zeros): it is no better than itself, yet its first position counts
-            v = m;
-            if (U * V == 1 || ifirst < 0) {
-#pragma unroll
-                for (int u = U - 1; u >= 0; --u)
-#pragma unroll
-                    for (int c = V - 1; c >= 0; --c) {
-                        const int32_t at = pos + u * step + c;
-                        if (u < n && e[u][c] == m && (unsigned)at < (unsigned)ifirst) ifirst = at;
-                    }
                 ilast = ifirst;
             }
         } else if (U * V == 1 && n && e[0][0] == m && m != 0.0f) {  // the ends of a segment come last
@@ -492,6 +549,29 @@ template <int W> __device__ __forceinline__ CSum lanes_csum(CSum a, unsigned mas
         const CSum b{__shfl_down_sync(mask, a.s, off), __shfl_down_sync(mask, a.c, off)};
         csum_merge(a, b);
     }
+    return a;
+}
+// The sums of W lanes, TWO or the first alone.  `check`: where lanes within the
+// float range are not together, again with every lane's share scaled.
+template <int W, bool TWO> __device__ __forceinline__ void lanes_sums(Sums &r, unsigned mask, bool check)
+{
+    const CSum a1 = r.s1, a2 = r.s2;
+    r.s1 = lanes_csum<W>(a1, mask);
+    if constexpr (TWO) r.s2 = lanes_csum<W>(a2, mask);
+    r.up = 1.0f;
+    if (!check) return;
+    bool out = !(r.s1.s - r.s1.s == 0.0f);
+    if constexpr (TWO) out |= !(r.s2.s - r.s2.s == 0.0f);
+    if (!__shfl_sync(mask, (int)out, (int)(threadIdx.x & 31 & ~(W - 1)))) return;  // (the first lane's are whole)
+    constexpr float down = 0x1p-64f;
+    r.up = 0x1p64f;
+    r.s1 = lanes_csum<W>(CSum{a1.s * down, a1.c * down}, mask);
+    if constexpr (TWO) r.s2 = lanes_csum<W>(CSum{a2.s * down, a2.c * down}, mask);
+}
+template <int W> __device__ __forceinline__ double lanes_sum64(double a, unsigned mask)
+{
+#pragma unroll
+    for (int off = W / 2; off; off >>= 1) a += __shfl_down_sync(mask, a, off);
     return a;
 }
 template <int W> __device__ __forceinline__ double lanes_prod(double a, unsigned mask)
@@ -564,6 +644,8 @@ __device__ __forceinline__ void ring_rows(float4 *ring, const float *at, int64_t
 // first and after the last multiple of 4 go element by element.  FINAL: one
 // chunk per segment; a block turns all its items into outputs at its end, a
 // thread each (FP64).  vec: the source is 16-byte addressable at multiples of 4.
+template <bool FIRST, class A, class B> struct Pick { typedef A type; };
+template <class A, class B> struct Pick<false, A, B> { typedef B type; };
 template <class Src, int OP, bool FINAL, bool IDX, int G>
 __device__ __forceinline__ void inner_body(const Src &src, int64_t inner, int64_t hi, int64_t chunk, int64_t q,
                                            int vec, Partial *__restrict__ part, float *__restrict__ out,
@@ -575,14 +657,17 @@ __device__ __forceinline__ void inner_body(const Src &src, int64_t inner, int64_
     constexpr int kBatch = Src::kBatch;
     constexpr bool kAsync = Src::kAsync && !EXT;  // (extremes look at a batch of all lanes)
     __shared__ float4 s_ring[kAsync ? kRing * kThreads : 1];
-    __shared__ Partial s_item[FINAL ? kItems : 1];
-    __shared__ Partial s_warp[2][kWarps];
+    static_assert(FINAL || G > 32, "chunks are a block's");
+    typedef typename Pick<(G > 32), Partial, Share>::type Item;
+    __shared__ Item s_item[FINAL ? kItems : 1];
+    __shared__ typename Pick<is_sum(OP), Share, Item>::type s_warp[2][kWarps];
     __shared__ float s_mean;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, tid = threadIdx.x % G;
     const unsigned mask = W == 32 ? 0xffffffffu : 0xffu << (lane & 24);
     const int64_t items = hi * q;
     const int per = (int)(((items + gridDim.x - 1) / gridDim.x + kGroups - 1) / kGroups) * kGroups;  // <= kItems
     const int64_t item0 = (int64_t)blockIdx.x * per;
+    const bool long_segment = G > 8 && chunk > 1024;  // (shorter ones are a warp's whole range anyhow)
     int turn = 0;
     for (int i = threadIdx.x / G; i < per && item0 + i < items; i += kGroups) {
         const int64_t item = item0 + i, seg = item / q, c = item - seg * q;
@@ -676,39 +761,65 @@ __device__ __forceinline__ void inner_body(const Src &src, int64_t inner, int64_
         };
         // the item's threads together; thread 0 of the item has the result.
         // (Two sets of shared slots in turn: a barrier an item is enough.)
-        Partial r;
+        Item r;
+        bool off = false;   // a variance: to be summed again, about
+        float mean = 0.0f;  // its mean
         auto together = [&]() {
-            if constexpr (is_var(OP)) {
-                r.v = var.sums();
-                r.v.s1 = lanes_csum<W>(r.v.s1, mask);
-                r.v.s2 = lanes_csum<W>(r.v.s2, mask);
-            } else if constexpr (is_sum(OP)) {
-                r.v.s1 = lanes_csum<W>(acc, mask);
-            } else if constexpr (OP == PROD) {
-                r.d = lanes_prod<W>(prod, mask);
-            } else {
-                r.b = run.best(k0, mask);
-            }
-            if constexpr (G > 32) {
-                if (lane == 0) s_warp[turn][wid] = r;
-                __syncthreads();
-                if (threadIdx.x < kWarps) {
-                    r = s_warp[turn][lane];
-                    constexpr unsigned few = (1u << kWarps) - 1;
-                    if constexpr (is_sum(OP)) r.v.s1 = lanes_csum<kWarps>(r.v.s1, few);
-                    if constexpr (is_var(OP)) r.v.s2 = lanes_csum<kWarps>(r.v.s2, few);
-                    if constexpr (OP == PROD) r.d = lanes_prod<kWarps>(r.d, few);
-                    if constexpr (EXT) r.b = lanes_best<MX, kWarps>(r.b, few);
+            if constexpr (is_sum(OP)) {
+                Share w;
+                if constexpr (is_var(OP)) w.v = var.sums();
+                else w.v.s1 = acc;
+                lanes_sums<W, is_var(OP)>(w.v, mask, long_segment);
+                if constexpr (G > 32) {
+                    if (lane == 0) s_warp[turn][wid] = w;
+                    __syncthreads();
+                    if (threadIdx.x < kWarps) {
+                        w = s_warp[turn][lane];
+                        constexpr unsigned few = (1u << kWarps) - 1;
+                        r.v.s1 = lanes_sum64<kWarps>(wide(w.v.s1, w.v.up), few);
+                        if constexpr (is_var(OP)) {
+                            r.v.s2 = lanes_sum64<kWarps>(wide(w.v.s2, w.v.up), few);
+                            r.v.piv = w.v.piv;
+                            off = VarAcc::off(r.v.s1, r.v.s2, k1 - k0);
+                            if (off) mean = (float)((double)w.v.piv + r.v.s1 / (double)(k1 - k0));
+                        }
+                    }
+                    turn ^= 1;
+                } else {
+                    r = w;
+                    if constexpr (is_var(OP)) {
+                        off = VarAcc::off(w.v, k1 - k0);
+                        mean = VarAcc::mean(w.v, k1 - k0);
+                    }
                 }
-                turn ^= 1;
+            } else {
+                if constexpr (EXT) r.b = run.best(k0, mask);
+                else r.d = lanes_prod<W>(prod, mask);
+                if constexpr (G > 32) {
+                    if (lane == 0) s_warp[turn][wid] = r;
+                    __syncthreads();
+                    if (threadIdx.x < kWarps) {
+                        r = s_warp[turn][lane];
+                        constexpr unsigned few = (1u << kWarps) - 1;
+                        if constexpr (EXT) r.b = lanes_best<MX, kWarps>(r.b, few);
+                        else r.d = lanes_prod<kWarps>(r.d, few);
+                    }
+                    turn ^= 1;
+                }
             }
         };
-        const float piv = is_var(OP) ? src.at(p0) : 0.0f;
-        if constexpr (is_var(OP)) var.start(piv, piv);
+        float piv = 0.0f;  // the mean of the first W elements, in every warp
+        if constexpr (is_var(OP)) {
+            const int few = k1 - k0 < W ? (int)(k1 - k0) : W, at = lane & (W - 1);
+            if (at < few) piv = __fdividef(src.at(p0 + at), (float)few);
+#pragma unroll
+            for (int off = W / 2; off; off >>= 1) piv += __shfl_xor_sync(mask, piv, off);
+            var.start(piv, piv);
+        }
         sweep();
         together();
         if constexpr (is_var(OP)) {
-            float mean = VarAcc::over(r.v) ? VarAcc::mean(r.v, k1 - k0) : piv;
+            if (!off) mean = piv;
             if constexpr (G > 32) {
                 if (threadIdx.x == 0) s_mean = mean;
                 __syncthreads();
@@ -716,14 +827,14 @@ __device__ __forceinline__ void inner_body(const Src &src, int64_t inner, int64_
             } else {
                 mean = __shfl_sync(mask, mean, lane & ~(W - 1));
             }
-            if (mean != piv && mean == mean) {
+            if (mean != piv && mean - mean == 0.0f) {
                 var.start(mean, mean);
                 sweep();
                 together();
             }
         }
         if (tid == 0) {
-            if (FINAL) s_item[i] = r;
+            if constexpr (FINAL) s_item[i] = r;
             else part[c * hi + seg] = r;
         }
     }
@@ -750,29 +861,38 @@ __device__ __forceinline__ void short_body(const Src &src, int64_t inner, int64_
         double prod = 1.0;
         Run<OP == MAX> run;
         VarAcc var;
-        if (is_var(OP)) var.start(src.at(base), src.at(base));
-        const float m = OP == MEANAD ? cen[seg] : 0.0f;
-        const float md = OP == MEANAD ? cen[hi + seg] : 0.0f;
-        for (int64_t k = 0; k < inner; ++k) {
-            const float v = src.at(base + k);
-            if (is_var(OP)) var.take(v);
-            else if (is_sum(OP)) sum_elem_c<OP>(acc, v, m, md);
-            else if (OP == PROD) prod *= (double)v;
-            else run.add(v, (int32_t)k);
-        }
-        if (is_var(OP)) {
-            Partial r;
+        auto sweep = [&](float piv) {
+            var.start(piv, piv);
+            int64_t k = 0;
+            for (; k + 2 <= inner; k += 2) var.take2(pk(src.at(base + k), src.at(base + k + 1)));
+            if (k < inner) var.take(src.at(base + k));
+        };
+        if constexpr (is_var(OP)) {
+            const int few = inner < 8 ? (int)inner : 8;
+            float piv = 0.0f;
+            for (int k = 0; k < few; ++k) piv += __fdividef(src.at(base + k), (float)few);
+            sweep(piv);
+            Share r;
             r.v = var.sums();
-            if (VarAcc::over(r.v)) {
-                const float mean = VarAcc::mean(r.v, inner);
-                var.start(mean, mean);
-                for (int64_t k = 0; k < inner; ++k) var.take(src.at(base + k));
+            const float mean = VarAcc::mean(r.v, inner);
+            if (VarAcc::off(r.v, inner) && mean - mean == 0.0f) {
+                sweep(mean);
                 r.v = var.sums();
             }
             Total<OP> t;
             t.add(r, (double)inner);
             t.put(out, index, out64, seg, hi, inner, cen);
-        } else if (is_sum(OP)) fold_put<OP>(out, out64, seg, hi, (double)acc.s + (double)acc.c, inner, cen);
+            continue;
+        }
+        const float m = OP == MEANAD ? cen[seg] : 0.0f;
+        const float md = OP == MEANAD ? cen[hi + seg] : 0.0f;
+        for (int64_t k = 0; k < inner; ++k) {
+            const float v = src.at(base + k);
+            if (is_sum(OP)) sum_elem_c<OP>(acc, v, m, md);
+            else if (OP == PROD) prod *= (double)v;
+            else run.add(v, (int32_t)k);
+        }
+        if (is_sum(OP)) fold_put<OP>(out, out64, seg, hi, (double)acc.s + (double)acc.c, inner, cen);
         else if (OP == PROD) { out[seg] = (float)prod; if (out64) out64[seg] = prod; }
         else {
             const Best b = run.to_best(0);
@@ -800,10 +920,10 @@ __device__ __forceinline__ void outer_body(const Src &src, int64_t lo, int64_t i
     constexpr int kWarps = kThreads / 32, kRows = Src::kBatch;
     constexpr bool kAsync = Src::kAsync && VEC == 4;
     // the rings, and then in their place the warps' partials
-    constexpr int kPartBytes = kWarps * 32 * VEC * (int)sizeof(Partial), kRingBytes = kAsync ? kRing * kThreads * 16 : 0;
+    constexpr int kPartBytes = kWarps * 32 * VEC * (int)sizeof(Share), kRingBytes = kAsync ? kRing * kThreads * 16 : 0;
     __shared__ __align__(16) char s_mem[kPartBytes > kRingBytes ? kPartBytes : kRingBytes];
     float4 *const s_ring = (float4 *)s_mem;
-    Partial(*const s_part)[32 * VEC] = (Partial(*)[32 * VEC])s_mem;
+    Share(*const s_part)[32 * VEC] = (Share(*)[32 * VEC])s_mem;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int64_t lv = lo / VEC;  // thread columns per h
     const int64_t c = blockIdx.y;
@@ -890,8 +1010,22 @@ __device__ __forceinline__ void outer_body(const Src &src, int64_t lo, int64_t i
             m[v] = OP == MEANAD && live ? cen[l + v + lo * h] : 0.0f;
             md[v] = OP == MEANAD && live ? cen[lo * hi + l + v + lo * h] : 0.0f;
         }
-        if constexpr (is_var(OP)) {
-            if (live) value(fetch(k0), k0, piv);
+        if constexpr (is_var(OP)) {  // the pivots: the mean of the warps' first rows
+            __shared__ float s_first[kWarps][32 * VEC];
+            const int few = k1 - k0 < kWarps ? (int)(k1 - k0) : kWarps;
+#pragma unroll
+            for (int v = 0; v < VEC; ++v) piv[v] = 0.0f;
+            if (live && wid < few) value(fetch(k0 + wid), k0 + wid, piv);
+#pragma unroll
+            for (int v = 0; v < VEC; ++v) {
+                s_first[wid][lane * VEC + v] = __fdividef(piv[v], (float)few);
+                piv[v] = 0.0f;
+            }
+            __syncthreads();
+#pragma unroll
+            for (int w = 0; w < kWarps; ++w)
+#pragma unroll
+                for (int v = 0; v < VEC; ++v) piv[v] += s_first[w][lane * VEC + v];
             start();
         }
         if (live) sweep();
@@ -900,11 +1034,9 @@ __device__ __forceinline__ void outer_body(const Src &src, int64_t lo, int64_t i
             if constexpr (kAsync) __syncthreads();  // (the partials take the rings' place)
 #pragma unroll
             for (int v = 0; v < VEC; ++v) {
-                Partial &r = s_part[wid][lane * VEC + v];
+                Share &r = s_part[wid][lane * VEC + v];
                 if constexpr (is_var(OP)) {
-                    const VarAcc &a = var[v / 2];
-                    r.v = Sums{CSum{VarAcc::half(a.s1, v & 1), VarAcc::half(a.c1, v & 1)},
-                               CSum{VarAcc::half(a.s2, v & 1), VarAcc::half(a.c2, v & 1)}, piv[v]};
+                    r.v = var[v / 2].sums(v & 1, piv[v]);
                 } else if constexpr (EXT) {
                     r.b = run[v].to_best(k0);
                 } else if constexpr (OP == PROD) {
@@ -915,17 +1047,51 @@ __device__ __forceinline__ void outer_body(const Src &src, int64_t lo, int64_t i
             }
             __syncthreads();
         };
+        bool off = false;   // a variance: to be summed again, about
+        float mean = 0.0f;  // its mean
         auto together = [&](int i) {
-            Partial r = s_part[0][i];
+            Partial r;
+            if constexpr (is_sum(OP)) {
+                Sum3 t1{s_part[0][i].v.s1}, t2{s_part[0][i].v.s2};
 #pragma unroll
-            for (int w = 1; w < kWarps; ++w) {
-                const Partial &o = s_part[w][i];
-                if constexpr (is_sum(OP)) csum_merge(r.v.s1, o.v.s1);
-                if constexpr (is_var(OP)) csum_merge(r.v.s2, o.v.s2);
-                if constexpr (OP == PROD) r.d *= o.d;
-                if constexpr (EXT) r.b = best_merge<MX>(r.b, o.b);
+                for (int w = 1; w < kWarps; ++w) {
+                    t1.add(s_part[w][i].v.s1);
+                    if constexpr (is_var(OP)) t2.add(s_part[w][i].v.s2);
+                }
+                r.v.s1 = t1.wide();
+                if constexpr (is_var(OP)) {
+                    r.v.s2 = t2.wide();
+                    r.v.piv = s_part[0][i].v.piv;
+                    const float n = (float)(k1 - k0), a = t1.s + t1.c, b = t2.s + t2.c;
+                    off = VarAcc::off(a, b, n);
+                    mean = r.v.piv + __fdividef(a, n);
+                }
+                if (!t1.in_range() || (is_var(OP) && !t2.in_range())) {  // warps within the float range are not together
+                    double s1 = 0.0, s2 = 0.0;
+                    for (int w = 0; w < kWarps; ++w) {
+                        s1 += wide(s_part[w][i].v.s1);
+                        if constexpr (is_var(OP)) s2 += wide(s_part[w][i].v.s2);
+                    }
+                    r.v.s1 = s1;
+                    if constexpr (is_var(OP)) {
+                        r.v.s2 = s2;
+                        off = VarAcc::off(s1, s2, k1 - k0);
+                        mean = (float)((double)r.v.piv + s1 / (double)(k1 - k0));
+                    }
+                }
+                return r;
+            } else {
+                const Share &o = s_part[0][i];
+                if constexpr (OP == PROD) r.d = o.d;
+                else r.b = o.b;
+#pragma unroll
+                for (int w = 1; w < kWarps; ++w) {
+                    const Share &o = s_part[w][i];
+                    if constexpr (OP == PROD) r.d *= o.d;
+                    else r.b = best_merge<MX>(r.b, o.b);
+                }
+                return r;
             }
-            return r;
         };
         give();
         const int i = threadIdx.x;
@@ -933,9 +1099,9 @@ __device__ __forceinline__ void outer_body(const Src &src, int64_t lo, int64_t i
         if (i < 32 * VEC) r = together(i);
         if constexpr (is_var(OP)) {
             __shared__ float s_mean[32 * VEC];
-            const bool over = i < 32 * VEC && VarAcc::over(r.v);
-            if (i < 32 * VEC) s_mean[i] = over ? VarAcc::mean(r.v, k1 - k0) : r.v.piv;
-            if (__syncthreads_or(over)) {
+            const bool again = i < 32 * VEC && off && mean - mean == 0.0f;
+            if (i < 32 * VEC) s_mean[i] = again ? mean : r.v.piv;
+            if (__syncthreads_or(again)) {
 #pragma unroll
                 for (int v = 0; v < VEC; ++v) piv[v] = s_mean[lane * VEC + v];
                 start();
