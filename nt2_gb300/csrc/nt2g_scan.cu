@@ -245,7 +245,9 @@ __global__ void __launch_bounds__(kLineThreads) k_scan_line(const float *x, int6
         begin = seg * inner + c * chunk;
         end = (c + 1) * chunk < inner ? begin + chunk : (seg + 1) * inner;
     }
-    SE<OP> carry = SE<OP>::id();  // warp 0's
+    // warp 0's: the elements before the tile, a sum's in FP64 (a pair of floats from
+    // the first tile to the last of a long segment would hold fewer bits)
+    ScanRec carry = rec_id<OP>();
     for (int64_t t0 = begin; t0 < end; t0 += kTile) {
         const int len = (int)(end - t0 < kTile ? end - t0 : kTile);
         const int mis = misalign(x + t0);
@@ -255,7 +257,7 @@ __global__ void __launch_bounds__(kLineThreads) k_scan_line(const float *x, int6
             const int64_t per = (c + kLineThreads - 1) / kLineThreads, i1 = (tid + 1) * per < c ? (tid + 1) * per : c;
             ScanRec p = rec_id<OP>();
             for (int64_t i = tid * per; i < i1; ++i) p = rec_combine<OP>(p, r[i]);
-            carry = from_rec<OP>(block_rec<OP>(p, s_rec));
+            carry = block_rec<OP>(p, s_rec);
         }
         tile_arrived();
         // PACK: a short tile still occupies every thread.  WALK runs past a
@@ -295,12 +297,21 @@ __global__ void __launch_bounds__(kLineThreads) k_scan_line(const float *x, int6
         if (lane == 0) { ex = SE<OP>::id(); exh = 0; }
         __syncthreads();
         if (wid == 0) {  // every warp's prefix, and the next tile's carry
-            SE<OP> pre = SE<OP>::id();
+            SE<OP> pre = SE<OP>::id(), upto = PACK ? SE<OP>::id() : from_rec<OP>(carry);
             for (int w = 0; w < kWarps; ++w) {
-                if (w == lane) pre = carry;
-                carry = PACK && whead[w] ? wtot[w] : SE<OP>::combine(carry, wtot[w]);
+                if (w == lane) pre = upto;
+                upto = PACK && whead[w] ? wtot[w] : SE<OP>::combine(upto, wtot[w]);
             }
             if (lane < kWarps) wpre[lane] = pre;
+            if (!PACK && t0 + kTile < end) {
+                if constexpr (OP == NT2G_SCAN_SUM) {
+                    upto = wtot[0];
+                    for (int w = 1; w < kWarps; ++w) upto = SE<OP>::combine(upto, wtot[w]);
+                    carry = rec_combine<OP>(carry, to_rec<OP>(upto));
+                } else {
+                    carry = to_rec<OP>(upto);
+                }
+            }
         }
         __syncthreads();
         SE<OP> run = PACK && exh ? ex : SE<OP>::combine(wpre[wid], ex);
