@@ -83,6 +83,16 @@ __global__ void __launch_bounds__(kFoldThreads, is_var(OP) ? 3 : 4) k_fold_outer
     outer_body<RawSrc, OP, VEC, FINAL>(src, lo, inner, hi, ck, q, part, out, index, cen, out64);
 }
 
+template <int OP, int VEC>
+__global__ void __launch_bounds__(kFoldThreads, is_var(OP) || OP == MEANAD ? 4 : VEC == 1 ? 8 : OP == MAX || OP == MIN ? 4 : 5) k_fold_columns(RawSrc src, int64_t lo, int64_t inner, int64_t hi,
+                                                             float *__restrict__ out, int64_t *__restrict__ index,
+                                                             const float *__restrict__ cen, double *__restrict__ out64)
+{
+    pdl_trigger();
+    pdl_wait_for(src.x, out, index, cen, out64);
+    columns_body<RawSrc, OP, VEC>(src, lo, inner, hi, out, index, cen, out64);
+}
+
 template <int OP>
 __global__ void __launch_bounds__(kFoldThreads) k_fold_nt2(RawSrc src, int64_t lo, int64_t inner, int64_t hi,
                                                            float *__restrict__ out, int64_t *__restrict__ index,
@@ -163,14 +173,32 @@ __global__ void __launch_bounds__(kFoldThreads) k_fold_finish_block(const Partia
 
 // --------------------------------------------------------------- plans --
 struct FoldPlan {
-    int kind = 0;       // 0 short segments, 1 contiguous (lo == 1), 2 strided
+    int kind = 0;       // 0 short segments, 1 contiguous (lo == 1), 2 strided, 3 strided with few rows
     int group = 0;      // contiguous: log2 of the threads per segment, as the index 0: 8, 1: 32, 2: 256
     int64_t chunk = 0;  // elements per chunk along the fold
     int64_t q = 1;      // chunks per output
     int vec = 0;
 };
 
-static FoldPlan plan_fold(int64_t lo, int64_t inner, int64_t hi, bool aligned, int op)
+// Whether a strided fold goes a thread per output, its rows one after the other
+// (columns_body), rather than shared out over a block's warps: few rows always,
+// more of them the more outputs there are to keep the GPU's loads in flight; more
+// than 31 rows only where a thread each fills the GPU, and not where the FP64 result
+// is asked for (a thread's sum is a pair of floats, what blocks hand on FP64).  Aligned rows (four outputs a thread; times
+// in us, warps and columns): 10^5 sums of 8 rows 4.4 and 2.2, of 24 5.2 and 3.6;
+// 4096 of 8 2.1 and 1.9, of 24 2.2 and 2.9; 2^20 of 64 53 and 40.  Others (one
+// output a thread, a warp's rows 128 bytes): 62000 sums of 24 rows 6.7 and 3.0,
+// maxima of 48 10.5 and 6.3; 301000 sums of 200 62.9 and 44.2.
+static bool by_columns(int64_t threads, int64_t inner, bool aligned, int op, bool want64)
+{
+    if (inner <= 8) return true;
+    if ((op == MAX || op == MIN) && !aligned && threads >= 49152 && inner <= 64) return true;
+    const bool many = threads >= 152 * 1024 && !want64;
+    if (aligned) return inner <= (many ? 64 : threads >= 16384 ? 31 : threads >= 4096 ? 20 : 8);
+    return inner <= (many ? 256 : threads >= 16384 ? 31 : 8);
+}
+
+static FoldPlan plan_fold(int64_t lo, int64_t inner, int64_t hi, bool aligned, int op, bool want64)
 {
     FoldPlan p;
     if (lo == 1) {
@@ -204,6 +232,11 @@ static FoldPlan plan_fold(int64_t lo, int64_t inner, int64_t hi, bool aligned, i
     }
     p.kind = 2;
     p.vec = aligned && (lo % 4 == 0) ? 4 : 1;
+    if (by_columns(lo * hi / p.vec, inner, p.vec == 4, op, want64)) {
+        p.kind = 3;
+        if (is_var(op)) p.vec = 1;  // (its FP64 ends keep a thread busy: more threads)
+        return p;
+    }
     const int64_t columns = (lo * hi / p.vec + 31) / 32;  // blocks side by side
     // (a variance's partials cost some twenty FP64 instructions each to combine)
     int64_t q = ((is_var(op) ? kBlocks / 2 : kBlocks) + columns - 1) / columns;
@@ -342,7 +375,7 @@ static nt2g_status launch_fold_op(const FoldInput &in, int64_t lo, int64_t inner
         if (ce != cudaSuccess) return cuda_status(ce, "fold launch");
         return NT2G_OK;
     }
-    FoldPlan p = plan_fold(lo, inner, hi, in.aligned, OP);
+    FoldPlan p = plan_fold(lo, inner, hi, in.aligned, OP, out64 != nullptr);
     if (p.q > 1 && (size_t)(n_out * p.q) * sizeof(Partial) > ws_bytes) {
         set_error("fold: workspace of %zu bytes, %zu needed", ws_bytes, (size_t)(n_out * p.q) * sizeof(Partial));
         return NT2G_ERR_INVALID;
@@ -383,6 +416,15 @@ static nt2g_status launch_fold_op(const FoldInput &in, int64_t lo, int64_t inner
         } else {
             void *pr[] = {(void *)jargs, &inner, &hi, &chunk, &q, &vec, &part, &out, &index, &cen, &out64};
             ce = launch_by_handle(jk->inner[fin ? p.group : 3][idx], g, pr, st);
+        }
+    } else if (p.kind == 3) {
+        const dim3 g(cap((n_out / p.vec + kFoldThreads - 1) / kFoldThreads));
+        if (!in.expr) {
+            if (!is_var(OP) && p.vec == 4) ce = launch_dependent(k_fold_columns<OP, is_var(OP) ? 1 : 4>, g, kFoldThreads, st, src, lo, inner, hi, out, index, cen, out64);
+            else ce = launch_dependent(k_fold_columns<OP, 1>, g, kFoldThreads, st, src, lo, inner, hi, out, index, cen, out64);
+        } else {
+            void *pr[] = {(void *)jargs, &lo, &inner, &hi, &out, &index, &cen, &out64};
+            ce = launch_by_handle(jk->columns[p.vec == 4], g, pr, st);
         }
     } else {
         const int64_t threads = n_out / p.vec;

@@ -199,10 +199,14 @@ struct Share {
         Best b;
     };
 };
-__device__ __forceinline__ double wide(const CSum &a, float up = 1.0f)
+__device__ __forceinline__ double wide(const CSum &a) { return (double)a.s + (double)a.c; }
+// times `up`, by the exponent's bits (a multiplication not needed costs as much of
+// the FP64 pipe as one that is)
+__device__ __forceinline__ double wide(const CSum &a, float up)
 {
-    const double t = (double)a.s + (double)a.c;
-    return up == 1.0f ? t : t * (double)up;
+    const double t = wide(a);
+    const int hi = __double2hiint(t), e = hi & 0x7ff00000;
+    return __hiloint2double(hi + (up != 1.0f && e != 0 && e != 0x7ff00000 ? 64 << 20 : 0), __double2loint(t));
 }
 // What a block hands on per (chunk, output), chunk-major: its warps together, in
 // FP64.
@@ -212,29 +216,6 @@ struct Partial {
         double d;
         Best b;
     };
-};
-
-// Three floats, each carrying the rounding errors of the one before: 72 bits, so
-// a block's warps combine with no fewer than FP64 has.  (An FP64 instruction
-// takes a warp sixteen cycles, however few of its lanes need it; the eight warps
-// of 128 outputs in FP64 would take 28 of them where this takes five.)
-struct Sum3 {
-    float s, c, d = 0.0f;
-    __device__ __forceinline__ explicit Sum3(const CSum &x) : s(x.s), c(x.c) {}
-    static __device__ __forceinline__ float two_sum(float &a, float b)
-    {
-        const float t = __fadd_rn(a, b), bb = __fsub_rn(t, a);
-        const float e = __fadd_rn(__fsub_rn(a, __fsub_rn(t, bb)), __fsub_rn(b, bb));
-        a = t;
-        return e;
-    }
-    __device__ __forceinline__ void add(const CSum &x)
-    {
-        const float e1 = two_sum(s, x.s), e2 = two_sum(c, x.c), e3 = two_sum(c, e1);
-        d = __fadd_rn(d, __fadd_rn(e2, e3));
-    }
-    __device__ __forceinline__ bool in_range() const { return s - s == 0.0f; }
-    __device__ __forceinline__ double wide() const { return (double)s + ((double)c + (double)d); }
 };
 
 // Chunks of one output combined in order.  A variance's sums are shifted to
@@ -260,17 +241,20 @@ template <int OP> struct Total {
             b = best_merge<OP == MAX>(b, p.b);
         }
     }
-    __device__ __forceinline__ void add(const Share &r, double n)
+    // the one share, or partial, of an output
+    __device__ __forceinline__ void set(const Share &r)
     {
-        Partial p;
-        if constexpr (is_sum(OP)) p.v.s1 = wide(r.v.s1, r.v.up);
-        if constexpr (is_var(OP)) {
-            p.v.s2 = wide(r.v.s2, r.v.up);
-            p.v.piv = r.v.piv;
-        }
-        if constexpr (OP == PROD) p.d = r.d;
-        if constexpr (!is_sum(OP) && OP != PROD) p.b = r.b;
-        add(p, n);
+        if constexpr (is_sum(OP)) t = wide(r.v.s1, r.v.up);
+        if constexpr (is_var(OP)) t2 = wide(r.v.s2, r.v.up);
+        if constexpr (OP == PROD) t = r.d;
+        if constexpr (!is_sum(OP) && OP != PROD) b = r.b;
+    }
+    __device__ __forceinline__ void set(const Partial &p)
+    {
+        if constexpr (is_sum(OP)) t = p.v.s1;
+        if constexpr (is_var(OP)) t2 = p.v.s2;
+        if constexpr (OP == PROD) t = p.d;
+        if constexpr (!is_sum(OP) && OP != PROD) b = p.b;
     }
     __device__ __forceinline__ void add(const Total &o, double n)  // n: the elements of o
     {
@@ -842,7 +826,7 @@ __device__ __forceinline__ void inner_body(const Src &src, int64_t inner, int64_
         __syncthreads();
         for (int i = threadIdx.x; i < per && item0 + i < items; i += kThreads) {
             Total<OP> t;
-            t.add(s_item[i], (double)inner);
+            t.set(s_item[i]);
             t.put(out, index, out64, item0 + i, hi, inner, cen);
         }
     }
@@ -880,7 +864,7 @@ __device__ __forceinline__ void short_body(const Src &src, int64_t inner, int64_
                 r.v = var.sums();
             }
             Total<OP> t;
-            t.add(r, (double)inner);
+            t.set(r);
             t.put(out, index, out64, seg, hi, inner, cen);
             continue;
         }
@@ -1052,7 +1036,7 @@ __device__ __forceinline__ void outer_body(const Src &src, int64_t lo, int64_t i
         auto together = [&](int i) {
             Partial r;
             if constexpr (is_sum(OP)) {
-                Sum3 t1{s_part[0][i].v.s1}, t2{s_part[0][i].v.s2};
+                Sum3 t1 = Sum3::of(s_part[0][i].v.s1), t2 = Sum3::of(s_part[0][i].v.s2);
 #pragma unroll
                 for (int w = 1; w < kWarps; ++w) {
                     t1.add(s_part[w][i].v.s1);
@@ -1115,13 +1099,126 @@ __device__ __forceinline__ void outer_body(const Src &src, int64_t lo, int64_t i
             const int64_t hh = ti / lv, o = (ti - hh * lv) * VEC + i % VEC + lo * hh;
             if (FINAL) {
                 Total<OP> t;
-                t.add(r, (double)inner);
+                t.set(r);
                 t.put(out, index, out64, o, lo * hi, inner, cen);
             } else {
                 part[c * (lo * hi) + o] = r;
             }
         }
         __syncthreads();
+    }
+}
+
+// Strided folds of a few rows: a thread per output (VEC: four neighbouring ones),
+// all its rows, a batch of them in flight.  (Rows shared out over a block's warps
+// leave most of those idle, and the block's steps cost more than the rows: ten
+// rows of 2^20 outputs, a sum and a maximum, 29 and 48 us so, 7.2 and 11 this way.)
+template <class Src, int OP, int VEC>
+__device__ __forceinline__ void columns_body(const Src &src, int64_t lo, int64_t inner, int64_t hi,
+                                             float *__restrict__ out, int64_t *__restrict__ index,
+                                             const float *__restrict__ cen, double *__restrict__ out64)
+{
+    constexpr bool MX = OP == MAX, EXT = OP == MAX || OP == MIN;
+    const int64_t lv = lo / VEC, n_out = lo * hi;
+    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < lv * hi; t += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t h = t / lv, l = (t - h * lv) * VEC, o = l + lo * h;
+        const int64_t base = l + lo * inner * h;
+        CSum acc[VEC];
+        double prod[VEC];
+        Run<MX> run[VEC];
+        VarAcc var[(VEC + 1) / 2];
+        float m[VEC], md[VEC], piv[VEC];
+        bool again = false;
+#pragma unroll
+        for (int v = 0; v < VEC; ++v) {
+            acc[v] = CSum{0.0f, 0.0f};
+            prod[v] = 1.0;
+            m[v] = OP == MEANAD ? cen[o + v] : 0.0f;
+            md[v] = OP == MEANAD ? cen[n_out + o + v] : 0.0f;
+        }
+        // rows k .. k + U
+        auto rows = [&](auto &e, int64_t k) {
+            constexpr int U = sizeof(e) / sizeof(e[0]);
+            typename Src::Raw raw[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                if constexpr (VEC == 4) raw[u] = src.fetch4(base + lo * (k + u));
+                else raw[u] = src.fetch(base + lo * (k + u));
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                if constexpr (VEC == 4) src.value4(raw[u], base + lo * (k + u), e[u]);
+                else e[u][0] = src.value(raw[u], base + lo * (k + u));
+            }
+            if constexpr (is_var(OP)) {
+                if (k == 0) {
+                    if (!again) {  // the pivots: the mean of the first rows
+#pragma unroll
+                        for (int v = 0; v < VEC; ++v) {
+                            piv[v] = 0.0f;
+#pragma unroll
+                            for (int u = 0; u < U; ++u) piv[v] += e[u][v] * (1.0f / U);
+                        }
+                    }
+#pragma unroll
+                    for (int v = 0; v < VEC; v += 2) var[v / 2].start(piv[v], piv[v + (VEC > 1)]);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+#pragma unroll
+                for (int v = 0; v < VEC; ++v) {
+                    if constexpr (is_var(OP)) {  // (VEC == 1: both halves the same)
+                        if (v % 2 == 0) var[v / 2].take2(pk(e[u][v], e[u][v + (VEC > 1)]));
+                    } else if constexpr (OP == PROD) {
+                        prod[v] *= (double)e[u][v];
+                    } else if constexpr (EXT) {
+                        run[v].add(e[u][v], (int32_t)(k + u));
+                    } else {
+                        sum_elem_c<OP>(acc[v], e[u][v], m[v], md[v]);
+                    }
+                }
+        };
+        do {
+            int64_t k = 0;
+            for (; k + Src::kBatch <= inner; k += Src::kBatch) {
+                float e[Src::kBatch][VEC];
+                rows(e, k);
+            }
+            for (; k < inner; ++k) {
+                float e[1][VEC];
+                rows(e, k);
+            }
+            if constexpr (is_var(OP)) {
+                if (again) break;
+#pragma unroll
+                for (int v = 0; v < VEC; ++v) {
+                    const Sums r = var[v / 2].sums(v & 1, piv[v]);
+                    const float mean = VarAcc::mean(r, inner);
+                    if (VarAcc::off(r, inner) && mean - mean == 0.0f) {
+                        piv[v] = mean;
+                        again = true;
+                    }
+                }
+            }
+        } while (again);
+#pragma unroll
+        for (int v = 0; v < VEC; ++v) {
+            if constexpr (OP == SUM || OP == ASUM1 || OP == ASUM2 || OP == NBTRUE || OP == NANSUM || OP == NOT_NAN) {
+                if (!out64) {  // rounded once, without an FP64 instruction
+                    out[o + v] = __fadd_rn(acc[v].s, acc[v].c);
+                    continue;
+                }
+            }
+            Share r;
+            if constexpr (is_var(OP)) r.v = var[v / 2].sums(v & 1, piv[v]);
+            else if constexpr (EXT) r.b = run[v].to_best(0);
+            else if constexpr (OP == PROD) r.d = prod[v];
+            else r.v = Sums{acc[v], acc[v], 0.0f, 1.0f};
+            Total<OP> total;
+            total.set(r);
+            total.put(out, index, out64, o + v, n_out, inner, cen);
+        }
     }
 }
 

@@ -102,13 +102,14 @@ nt2g_status launch_fold_expr(const std::vector<nt2g_op> &ops, const std::vector<
 // Fold kernels of a program with a FOLD instruction: the first-phase kernels
 // of nt2g_fold_kernels.cuh (NT2-order, short-segment, contiguous
 // inner[8 | 32 | 256 threads a segment | 256 a chunk][IDX], strided
-// outer[VEC == 4][FINAL]) instantiated over the program's element
+// outer[VEC == 4][FINAL] and columns[VEC == 4]) instantiated over the program's element
 // function, for one fold op; nullptr, with the reason in *why, when NVRTC is
 // unavailable or rejects the source.
 struct JitFoldKernels {
     cudaKernel_t nt2 = nullptr, shrt = nullptr;
     cudaKernel_t inner[4][2] = {};
     cudaKernel_t outer[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};
+    cudaKernel_t columns[2] = {nullptr, nullptr};
 };
 const JitFoldKernels *jit_fold_kernels(const std::vector<nt2g_op> &ops, const std::vector<uint8_t> &logical,
                                        int precision, int op, std::string *why);

@@ -522,6 +522,11 @@ std::string jit_fold_source(const std::vector<nt2g_op> &ops, const std::vector<u
                  "{ nt2g::fold::outer_body<ExprSrc, NT2G_FOP, " + V + ", " + F +
                  ">(ExprSrc{a}, lo, inner, hi, ck, q, part, out, index, cen, out64); }\n";
         }
+    for (int v4 = 0; v4 < 2; ++v4)
+        s += "extern \"C\" __global__ void __launch_bounds__(256) fold_columns_" + std::to_string(v4) +
+             "(const JitArgs a, long long lo, long long inner, long long hi, float *out, long long *index, const float *cen, "
+             "double *out64)\n{ nt2g::fold::columns_body<ExprSrc, NT2G_FOP, " + (v4 ? "4" : "1") +
+             ">(ExprSrc{a}, lo, inner, hi, out, index, cen, out64); }\n";
     return s;
 }
 
@@ -1118,6 +1123,9 @@ const JitFoldKernels *jit_fold_kernels(const std::vector<nt2g_op> &ops, const st
                         if (ce == cudaSuccess)
                             ce = cudaLibraryGetKernel(&e.k.outer[a][b], e.lib,
                                                       ("fold_outer_" + std::to_string(a) + std::to_string(b)).c_str());
+                for (int a = 0; a < 2; ++a)
+                    if (ce == cudaSuccess)
+                        ce = cudaLibraryGetKernel(&e.k.columns[a], e.lib, ("fold_columns_" + std::to_string(a)).c_str());
             }
             if (ce == cudaSuccess) {
                 e.ok = true;
