@@ -845,16 +845,26 @@ __device__ __forceinline__ void short_body(const Src &src, int64_t inner, int64_
         double prod = 1.0;
         Run<OP == MAX> run;
         VarAcc var;
-        auto sweep = [&](float piv) {
-            var.start(piv, piv);
-            int64_t k = 0;
-            for (; k + 2 <= inner; k += 2) var.take2(pk(src.at(base + k), src.at(base + k + 1)));
-            if (k < inner) var.take(src.at(base + k));
-        };
         if constexpr (is_var(OP)) {
-            const int few = inner < 8 ? (int)inner : 8;
-            float piv = 0.0f;
-            for (int k = 0; k < few; ++k) piv += __fdividef(src.at(base + k), (float)few);
+            // the first elements stay in registers: their mean is the pivot
+            constexpr int F = 8;
+            const int few = inner < F ? (int)inner : F;
+            float e[F], piv = 0.0f;
+#pragma unroll
+            for (int u = 0; u < F; ++u) e[u] = u < few ? src.at(base + u) : 0.0f;
+#pragma unroll
+            for (int u = 0; u < F; ++u) piv += __fdividef(e[u], (float)few);
+            auto sweep = [&](float piv) {
+                var.start(piv, piv);
+#pragma unroll
+                for (int u = 0; u < F; u += 2) {
+                    if (u + 2 <= few) var.take2(pk(e[u], e[u + 1]));
+                    else if (u < few) var.take(e[u]);
+                }
+                int64_t k = F;
+                for (; k + 2 <= inner; k += 2) var.take2(pk(src.at(base + k), src.at(base + k + 1)));
+                if (k < inner) var.take(src.at(base + k));
+            };
             sweep(piv);
             Share r;
             r.v = var.sums();
