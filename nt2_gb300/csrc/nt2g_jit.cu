@@ -850,8 +850,8 @@ constexpr size_t kVjpRing = 8;  // 2 x 8 x 256 x 8 bytes: 32 KB
 // output slot with that slot's cotangent table, runs the adjoint rules in
 // reverse instruction order, and writes the adjoints of the loaded values to
 // the slots' gradient tables.  Adjoints of float scalars are summed per
-// thread (vjp::ScalarSum), then per block in FP64 (fixed order) into
-// partials[block][scalar].
+// thread (vjp::ScalarSum), then per warp in three floats and per block in FP64
+// (fixed order) into partials[block][scalar].
 std::string jit_vjp_source(const std::vector<nt2g_op> &ops, const std::vector<uint8_t> &logical, int precision,
                            std::string *why)
 {
@@ -965,15 +965,25 @@ std::string jit_vjp_source(const std::vector<nt2g_op> &ops, const std::vector<ui
     if (ring)
         s += "    if (vec) {\n"
              "        __shared__ float2 r[2][" + std::to_string(rows.size()) + "][256];\n"
-             "        ring_fill(r[0], a, g, i, n);\n"
-             "        ring_fill(r[1], a, g, i + stride, n);\n"
-             "        for (int t = 0; i + 2 <= n; i += stride, t ^= 1) {\n"
+             "        JitIn in;\n"
+             "        if (n <= stride) {\n"  // (one pair a thread: directly)
+             "            if (i + 2 <= n) jit_fetch<true>(a, g, i, 2, in);\n"
+             "        } else {\n"
+             "            ring_fill(r[0], a, g, i, n);\n"
+             "            ring_fill(r[1], a, g, i + stride, n);\n"
              "            asm volatile(\"cp.async.wait_group 1;\" ::: \"memory\");\n"
-             "            JitIn in;\n"
+             "            ring_read(r[0], in);\n"
+             "            if (i + 2 <= n) jit_bytes<true>(a, i, 2, in);\n"
+             "        }\n"
+             "        for (int t = 0; i + 2 <= n;) {\n"
+             "            vjp_tile<P, true>(a, g, in, i, 2, sacc);\n"
+             "            i += stride;\n"
+             "            if (i + 2 > n) break;\n"
+             "            ring_fill(r[t], a, g, i + stride, n);\n"
+             "            t ^= 1;\n"
+             "            asm volatile(\"cp.async.wait_group 1;\" ::: \"memory\");\n"
              "            ring_read(r[t], in);\n"
              "            jit_bytes<true>(a, i, 2, in);\n"
-             "            vjp_tile<P, true>(a, g, in, i, 2, sacc);\n"
-             "            ring_fill(r[t], a, g, i + 2 * stride, n);\n"
              "        }\n"
              "    }\n";
     s += "    for (; i < n; i += stride) {\n"
@@ -989,18 +999,21 @@ std::string jit_vjp_source(const std::vector<nt2g_op> &ops, const std::vector<ui
          "        vjp_tile<P, false>(a, g, in, i, cnt, sacc);\n"
          "    }\n";
     if (ns > 0)
-        s += "    __shared__ double red[8][NT2G_NS];\n"
+        s += "    __shared__ nt2g::Sum3 red[NT2G_NS][8];\n"
+             "    __shared__ double red_far[NT2G_NS][8];\n"
+             "    if (!partials) return;\n"
              "    for (int q = 0; q < NT2G_NS; ++q) {\n"
-             "        double x = sacc[q].total();\n"
-             "        for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);\n"
-             "        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5][q] = x;\n"
+             "        const nt2g::Sum3 x = sacc[q].warp();\n"
+             "        const double far = sacc[q].warp_far();\n"
+             "        if ((threadIdx.x & 31) == 0) { red[q][threadIdx.x >> 5] = x; red_far[q][threadIdx.x >> 5] = far; }\n"
              "    }\n"
              "    __syncthreads();\n"
-             "    if (partials && threadIdx.x < NT2G_NS) {\n"
-             "        double x = 0.0;\n"
-             "        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) x += red[w][threadIdx.x];\n"
-             "        partials[(long long)blockIdx.x * NT2G_NS + threadIdx.x] = x;\n"
-             "    }\n";
+             "    for (int q = threadIdx.x >> 5; q < NT2G_NS; q += 8)\n"
+             "        if ((threadIdx.x & 31) < 8) {\n"
+             "            double x = red[q][threadIdx.x & 7].wide() + red_far[q][threadIdx.x & 7];\n"
+             "            for (int o = 4; o > 0; o >>= 1) x += __shfl_down_sync(0xffu, x, o);\n"
+             "            if ((threadIdx.x & 31) == 0) partials[(long long)blockIdx.x * NT2G_NS + q] = x;\n"
+             "        }\n";
     s += "}\n";
     return s;
 }
@@ -1243,11 +1256,12 @@ static JitVjpEntry *jit_vjp_get(const std::vector<nt2g_op> &ops, const std::vect
     return &it->second;
 }
 
-// Blocks of the reverse-mode grid: 256 threads x 4 elements each, at most
-// 8 resident blocks (2048 threads) per SM.
-static int64_t vjp_grid_bound(int64_t count)
+// Blocks of the reverse-mode grid that hands on scalars' sums: 256 threads of a
+// pair of elements each, at most 8 (2048 threads) per SM, which also ends the
+// second wave of programs of more than four resident blocks there.
+static int64_t vjp_grid_bound(int64_t count, int64_t per_block = 512)
 {
-    const int64_t need = (count + 1023) / 1024;
+    const int64_t need = (count + per_block - 1) / per_block;
     const int64_t full = (int64_t)device_sm_count() * 8;
     return need < full ? need : full;
 }
@@ -1308,14 +1322,20 @@ nt2g_status launch_vjp(const std::vector<nt2g_op> &ops, const std::vector<uint8_
     // pairs or more (2^24 elements: 167 us with one wave, 162 with two; 2^20: 14.0
     // and 15.3, the blocks' scalar sums included)
     if (count >= full * 2 * 256 * 2 * 8) full *= 2;
-    const int grid = (int)(bound < full ? bound : full);
+    const bool sums = scalar_grads && ns > 0;
+    const int64_t need = sums ? bound : (count + 511) / 512;
+    if (!sums && need < 2 * full) full = need;  // (less than two passes: a block for every 512 elements)
+    int grid = (int)(need < full ? need : full);
     double *partials = nullptr;
-    if (scalar_grads && ns > 0) {
-        const size_t need = (size_t)grid * ns * sizeof(double);
-        if (!ws || ws_bytes < need || ((uintptr_t)ws & 7u)) {
-            set_error("nt2g_program_vjp: workspace of %zu bytes, %zu needed (8-byte aligned)", ws_bytes, need);
+    if (sums) {
+        // (a workspace for half the blocks will do: threads with two pairs each)
+        const int64_t half = vjp_grid_bound(count, 1024);
+        const size_t least = (size_t)(half < full ? half : full) * ns * sizeof(double);
+        if (!ws || ws_bytes < least || ((uintptr_t)ws & 7u)) {
+            set_error("nt2g_program_vjp: workspace of %zu bytes, %zu needed (8-byte aligned)", ws_bytes, least);
             return NT2G_ERR_INVALID;
         }
+        if ((size_t)grid * ns * sizeof(double) > ws_bytes) grid = (int)(ws_bytes / (ns * sizeof(double)));
         partials = (double *)ws;
     }
     struct { const float *ct[kMaxSlots]; float *grad[kMaxSlots]; } g;
