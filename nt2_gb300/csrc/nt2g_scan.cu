@@ -39,7 +39,14 @@ constexpr int kLineThreads = 128, kRun = 33;       // contiguous tiles: 128 thre
 constexpr int kTileMax = kLineThreads * kRun;      // 17 KB of shared memory, 13 blocks an SM
 constexpr int64_t kPackBelow = 1024;               // segments shorter than this share tiles
 constexpr int64_t kLineChunks = 152 * 12;          // chunks (blocks) a contiguous scan is cut into at least
-constexpr int64_t kInlinePrefix = 64;              // strided chunks whose prefix the scan itself adds up
+// strided chunks whose prefix the scan itself adds up: every thread reads the records
+// above it, which with four segments a thread costs more than one more kernel from
+// eight chunks on (running maxima of 4096 columns of 100, 128, 256 and 1024 rows, us:
+// 9.0, 11.1, 16.6, 49.0 so; 11.7, 9.4, 10.8, 20.0 with the kernel), with one segment
+// a thread not (4099 columns of 250, 1000 and 8190: 7.3, 14.7, 79.6; 10.6, 18.4,
+// 86.6), but for the maxima of too few segments to hide a chain of compares (31 of
+// 512 and 1024: 9.2, 14.7; 7.2, 10.2)
+constexpr int64_t kInlineFew = 7, kInlinePrefix = 64;
 constexpr int64_t kScanTarget = 152 * 1024;
 
 // ------------------------------------------------------------- elements --
@@ -423,8 +430,15 @@ __global__ void __launch_bounds__(kLineThreads) k_scan_fold(const float *__restr
 // chunk [c*ck, min((c+1)*ck, inner)) of the scan range; grid.y = chunk.
 // FOLD: the chunk's aggregate.  Else the scan, from the aggregates of the chunks above (`prefixes`: k_scan_prefix* has
 // replaced them by their sums).
+// k rows in groups, the last ones in smaller ones (running sums of ten rows of 3.3
+// million segments: 126 us with the last ones one at a time, 57 so)
+#define NT2G_GROUPS                                                 \
+    while (k >= kGroup) { float e[kGroup][VEC]; group(e); }         \
+    if (kGroup > 8 && k >= 8) { float e[8][VEC]; group(e); }        \
+    if (kGroup > 4 && k >= 4) { float e[4][VEC]; group(e); }        \
+    while (k > 0) { float e[1][VEC]; group(e); }
 template <int OP, int VEC, bool FOLD>
-__global__ void __launch_bounds__(kScanThreads) k_scan_outer(const float *x, int64_t lo, int64_t inner, int64_t hi,
+__global__ void __launch_bounds__(kScanThreads, VEC == 4 ? 4 : 0) k_scan_outer(const float *x, int64_t lo, int64_t inner, int64_t hi,
                                                              int64_t ck, int64_t q, bool prefixes,
                                                              ScanRec *__restrict__ rec, float *out)
 {
@@ -461,21 +475,17 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_outer(const float *x, int
         if constexpr (FOLD) {
             const float *p = x + base + lo * k0;
             int64_t k = k1 - k0;
-            for (; k >= kGroup; k -= kGroup) {
-                float e[kGroup][VEC];
+            auto group = [&](auto &e) {
+                constexpr int G = sizeof(e) / sizeof(e[0]);
 #pragma unroll
-                for (int g = 0; g < kGroup; ++g, p += lo) fetch(p, e[g]);
+                for (int g = 0; g < G; ++g, p += lo) fetch(p, e[g]);
 #pragma unroll
-                for (int g = 0; g < kGroup; ++g)
+                for (int g = 0; g < G; ++g)
 #pragma unroll
                     for (int v = 0; v < VEC; ++v) carry[v].push(e[g][v]);
-            }
-            for (; k > 0; --k, p += lo) {
-                float e[VEC];
-                fetch(p, e);
-#pragma unroll
-                for (int v = 0; v < VEC; ++v) carry[v].push(e[v]);
-            }
+                k -= G;
+            };
+            NT2G_GROUPS
 #pragma unroll
             for (int v = 0; v < VEC; ++v) rec[c * n_seg + (l + v + lo * h)] = to_rec<OP>(carry[v]);
         } else {
@@ -493,18 +503,15 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_outer(const float *x, int
                 o += lo;
             };
             int64_t k = k1 - k0;
-            for (; k >= kGroup; k -= kGroup) {
-                float e[kGroup][VEC];
+            auto group = [&](auto &e) {
+                constexpr int G = sizeof(e) / sizeof(e[0]);
 #pragma unroll
-                for (int g = 0; g < kGroup; ++g, p += lo) fetch(p, e[g]);
+                for (int g = 0; g < G; ++g, p += lo) fetch(p, e[g]);
 #pragma unroll
-                for (int g = 0; g < kGroup; ++g) step(e[g]);
-            }
-            for (; k > 0; --k, p += lo) {
-                float e[VEC];
-                fetch(p, e);
-                step(e);
-            }
+                for (int g = 0; g < G; ++g) step(e[g]);
+                k -= G;
+            };
+            NT2G_GROUPS
         }
     }
 }
@@ -730,9 +737,14 @@ static nt2g_status launch_scan_op(const float *x, int64_t lo, int64_t inner, int
 #undef NT2G_LINE
         }
     } else {
-        const dim3 grid(cap((n_seg / p.vec + kScanThreads - 1) / kScanThreads), (unsigned)p.q);
-        const bool prefixes = p.q > kInlinePrefix;
-#define NT2G_OUTER(VEC, FOLD) k_scan_outer<OP, VEC, FOLD><<<grid, kScanThreads, 0, st>>>(x, lo, inner, hi, p.chunk, p.q, \
+        // blocks no wider than the segments are many (an SM holds eight of 256 threads,
+        // whatever few of them have a segment)
+        const int64_t threads = n_seg / p.vec;
+        const int block = threads < kScanThreads ? (int)((threads + 31) / 32 * 32) : kScanThreads;
+        const dim3 grid(cap((threads + kScanThreads - 1) / kScanThreads), (unsigned)p.q);
+        const bool few = p.vec == 4 || ((OP == NT2G_SCAN_MAX || OP == NT2G_SCAN_MIN) && n_seg < 1024);
+        const bool prefixes = p.q > (few ? kInlineFew : kInlinePrefix);
+#define NT2G_OUTER(VEC, FOLD) k_scan_outer<OP, VEC, FOLD><<<grid, block, 0, st>>>(x, lo, inner, hi, p.chunk, p.q, \
                                                                                          prefixes, rec, out)
         if (p.q > 1) {
             if (p.vec == 4) NT2G_OUTER(4, true);
