@@ -414,12 +414,17 @@ nt2g_status launch_bs(const float *S, const float *K, const float *T, const floa
     const int64_t exact_grid = ((n >> 2) + threads - 1) / threads > 0 ? ((n >> 2) + threads - 1) / threads : 1;
     // launched while the stream's previous kernel still runs (its blocks wait for it
     // to end), so a stream of calls has no gap between kernels: 2^20 options a call
-    // 8.2 us, now 5.3, the host's time; 3M under the NT2 policy 30.7, now 27.9
+    // 8.2 us, now 5.3, the host's time; 3M under the NT2 policy 30.7, now 27.9.  Not
+    // where a grid is a part of a wave: the next one's blocks would settle on the SMs
+    // that finish first, several to one (300 000 options 2.9 us and 3.7 lined up,
+    // under the NT2 policy 4.5 and 5.9; 10^5 and 622 592 no slower lined up)
+    const bool in_turn = threads == 256 && exact_grid > 152 && exact_grid < 152 * 4;
     cudaError_t ce = cudaSuccess;
 #define NT2G_BS(PP, TAB)                                                                                       \
     do {                                                                                                       \
-        if (vec) ce = launch_dependent(k_bs<PP, TAB, true>, dim3((unsigned)exact_grid), threads, st, S, K, T, sig,  \
-                                       sig_s, r, call, put, n);                                                \
+        if (vec && in_turn) k_bs<PP, TAB, true><<<(unsigned)exact_grid, threads, 0, st>>>(S, K, T, sig, sig_s, r, call, put, n); \
+        else if (vec) ce = launch_dependent(k_bs<PP, TAB, true>, dim3((unsigned)exact_grid), threads, st, S, K, T, sig,  \
+                                            sig_s, r, call, put, n);                                           \
         else k_bs<PP, TAB, false><<<grid_for(k_bs<PP, TAB, false>, n), 256, 0, st>>>(S, K, T, sig, sig_s, r,   \
                                                                                       call, put, n);           \
     } while (0)
