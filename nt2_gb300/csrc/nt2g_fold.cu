@@ -84,7 +84,7 @@ __global__ void __launch_bounds__(kFoldThreads, is_var(OP) ? 3 : 4) k_fold_outer
 }
 
 template <int OP, int VEC>
-__global__ void __launch_bounds__(kFoldThreads, is_var(OP) || OP == MEANAD ? 4 : VEC == 1 ? 8 : OP == MAX || OP == MIN ? 4 : 5) k_fold_columns(RawSrc src, int64_t lo, int64_t inner, int64_t hi,
+__global__ void __launch_bounds__(kFoldThreads, VEC == 4 || is_var(OP) || OP == MEANAD ? 4 : 8) k_fold_columns(RawSrc src, int64_t lo, int64_t inner, int64_t hi,
                                                              float *__restrict__ out, int64_t *__restrict__ index,
                                                              const float *__restrict__ cen, double *__restrict__ out64)
 {
