@@ -428,8 +428,8 @@ __global__ void __launch_bounds__(kLineThreads) k_scan_fold(const float *__restr
 // ---------------------------------------------- strided scans (lo > 1) --
 // Thread per segment (VEC: four neighbouring segments via float4) over the
 // chunk [c*ck, min((c+1)*ck, inner)) of the scan range; grid.y = chunk.
-// FOLD: the chunk's aggregate.  Else the scan, from the aggregates of the chunks above (`prefixes`: k_scan_prefix* has
-// replaced them by their sums).
+// FOLD: the chunk's aggregate (KEEP: leaving the table in L2).  Else the scan, from the aggregates of the chunks above
+// (`prefixes`: k_scan_prefix* has replaced them by their sums).
 // k rows in groups, the last ones in smaller ones (running sums of ten rows of 3.3
 // million segments: 126 us with the last ones one at a time, 57 so)
 #define NT2G_GROUPS                                                 \
@@ -437,7 +437,7 @@ __global__ void __launch_bounds__(kLineThreads) k_scan_fold(const float *__restr
     if (kGroup > 8 && k >= 8) { float e[8][VEC]; group(e); }        \
     if (kGroup > 4 && k >= 4) { float e[4][VEC]; group(e); }        \
     while (k > 0) { float e[1][VEC]; group(e); }
-template <int OP, int VEC, bool FOLD>
+template <int OP, int VEC, bool FOLD, bool KEEP = true>
 __global__ void __launch_bounds__(kScanThreads, VEC == 4 ? 4 : 0) k_scan_outer(const float *x, int64_t lo, int64_t inner, int64_t hi,
                                                              int64_t ck, int64_t q, bool prefixes,
                                                              ScanRec *__restrict__ rec, float *out)
@@ -466,7 +466,7 @@ __global__ void __launch_bounds__(kScanThreads, VEC == 4 ? 4 : 0) k_scan_outer(c
         }
         auto fetch = [&](const float *p, float (&e)[VEC]) {
             if constexpr (VEC == 4) {
-                const float4 f = FOLD ? __ldg((const float4 *)p) : ld_stream((const float4 *)p);
+                const float4 f = FOLD && KEEP ? __ldg((const float4 *)p) : ld_stream((const float4 *)p);
                 e[0] = f.x; e[1] = f.y; e[2] = f.z; e[3] = f.w;
             } else {
                 e[0] = FOLD ? __ldg(p) : ld_stream(p);
@@ -742,13 +742,18 @@ static nt2g_status launch_scan_op(const float *x, int64_t lo, int64_t inner, int
         const int64_t threads = n_seg / p.vec;
         const int block = threads < kScanThreads ? (int)((threads + 31) / 32 * 32) : kScanThreads;
         const dim3 grid(cap((threads + kScanThreads - 1) / kScanThreads), (unsigned)p.q);
+        // the fold leaves in L2 what the scan reads again where that fits (running maxima
+        // of 4096 x 4096 51 us, 56 with streaming loads; of 16384 x 16384 515 and 501;
+        // single columns, whose warps share sectors, always: 4099 x 8190 80 and 165)
+        const bool keep = n_seg * inner <= (int64_t)24 << 20;
         const bool few = p.vec == 4 || ((OP == NT2G_SCAN_MAX || OP == NT2G_SCAN_MIN) && n_seg < 1024);
         const bool prefixes = p.q > (few ? kInlineFew : kInlinePrefix);
-#define NT2G_OUTER(VEC, FOLD) k_scan_outer<OP, VEC, FOLD><<<grid, block, 0, st>>>(x, lo, inner, hi, p.chunk, p.q, \
+#define NT2G_OUTER(VEC, ...) k_scan_outer<OP, VEC, __VA_ARGS__><<<grid, block, 0, st>>>(x, lo, inner, hi, p.chunk, p.q, \
                                                                                          prefixes, rec, out)
         if (p.q > 1) {
-            if (p.vec == 4) NT2G_OUTER(4, true);
-            else NT2G_OUTER(1, true);
+            if (p.vec != 4) NT2G_OUTER(1, true);
+            else if (keep) NT2G_OUTER(4, true);
+            else NT2G_OUTER(4, true, false);
             if (prefixes) launch_prefix<OP>(rec, n_seg, p.q, st);
         }
         if (p.vec == 4) NT2G_OUTER(4, false);
