@@ -206,31 +206,34 @@ static FoldPlan plan_fold(int64_t lo, int64_t inner, int64_t hi, bool aligned, i
         p.kind = 1;
         p.vec = aligned;
         // at least 32 elements (eight float4 loads) a thread, with more threads a
-        // segment where there are too few segments to fill the GPU, and at most 512:
-        // a thread's sum is a pair of floats, what it hands on FP64 within a warp
+        // segment where there are too few segments to fill the GPU, and at most 512 of
+        // a sum's: a thread holds a pair of floats, what it hands on FP64 within a warp
         // (us, sums: 4000 of 65 elements 3.8 by 32 threads, 2.4 by 8; 16000 of 257 8.7
         // and 5.2; 838 of 600 4.1 by 256, 3.1 by 32; 3000 of 2049 12.9 by 256, 5.7 by 32)
         p.group = inner <= (hi < 152 * 8 ? 64 : hi < 152 * 32 ? 128 : hi < 152 * 64 ? 256 : 640) ? 0 : 1;
         if (p.group == 1 && inner > 512 &&
             hi < (inner <= 1024 ? 152 * 4 : inner < 4096 ? 152 * 8 : inner < 8192 ? 152 * 12 : 152 * 16))
             p.group = 2;
-        if (inner > kMostPerThread * 32) p.group = 2;
+        const int64_t most = is_sum(op) ? kMostPerThread : (int64_t)1 << 20;
+        if (inner > most * 32) p.group = 2;
         p.chunk = inner > 0 ? inner : 1;
-        if (p.group == 2 && (hi < kBlocks || inner > kMostPerThread * kFoldThreads)) {
+        if (p.group == 2 && (hi < kBlocks || inner > most * kFoldThreads)) {
             // one wave of four blocks an SM for a few long segments (2^24 elements:
             // a sum of exponentials and a maximum 26.0 and 16.9 us in 1824 blocks,
             // 22.3 and 13.2 in 608, 27.1 and 15.8 in 912; their partials 12.2 us to
             // combine, now 7.3); more, and shorter, blocks for more segments and for
             // tables far larger than the L2 cache, where the wave's last blocks cost
             // more than that (10^8 elements: 120 and 118 us)
-            const int64_t per = hi <= kWave / 2 && inner * hi <= 1 << 25 ? kWave / hi : (kBlocks + hi - 1) / hi;
+            int64_t per = hi <= kWave / 2 && inner * hi <= 1 << 25 ? kWave / hi : (kBlocks + hi - 1) / hi;
+            // (waves more where chunks would be too long, not part of one: 2^28 elements,
+            // a sum of exponentials 8.5e11 elements/s in four waves, 8.2e11 in 3.4)
+            while (per * most * kFoldThreads < inner) per += (kWave + hi - 1) / hi;
             int64_t chunk = (inner + per - 1) / per;
             if (chunk < 4096) chunk = 4096;
             // one chunk, and no kernel to combine its partials, for short segments, and
             // for longer ones the more of them there are (us: 838 sums of 5000 9.1 in two
             // chunks each, 5.4 in one; 10 of them 4.4 and 2.4; 838 of 17000 14.1 and 8.6)
             if (inner < 8192 || (hi >= kWave / 2 && inner < 32768)) chunk = inner;
-            if (chunk > kMostPerThread * kFoldThreads) chunk = kMostPerThread * kFoldThreads;
             p.chunk = (chunk + 1023) / 1024 * 1024;
             p.q = (inner + p.chunk - 1) / p.chunk;
             if (p.q < 1) p.q = 1;

@@ -55,9 +55,11 @@
 #include "nt2g_f2.cuh"
 #define NT2G_FOLD_INF __builtin_huge_valf()
 #define NT2G_FOLD_NAN __builtin_nanf("")
+#define NT2G_FOLD_SELDOM __forceinline__
 #else
 #define NT2G_FOLD_INF __int_as_float(0x7f800000)
 #define NT2G_FOLD_NAN __int_as_float(0x7fffffff)
+#define NT2G_FOLD_SELDOM __noinline__
 #endif
 
 namespace nt2g {
@@ -536,7 +538,17 @@ template <int W> __device__ __forceinline__ CSum lanes_csum(CSum a, unsigned mas
     return a;
 }
 // The sums of W lanes, TWO or the first alone.  `check`: where lanes within the
-// float range are not together, again with every lane's share scaled.
+// float range are not together, again with every lane's share scaled -- in folds of
+// expressions by a call, seldom made: inline it took registers from their loads
+// (sum(abs(x - y), 1) of 16384 squared 7.5e11 elements/s, 8.6e11 so; a table's, sum(A,
+// 1) of the same size, 1.76e12 inline and 1.71e12 by a call).
+template <int W, bool TWO> __device__ NT2G_FOLD_SELDOM void lanes_scaled(Sums &r, CSum a1, CSum a2, unsigned mask)
+{
+    constexpr float down = 0x1p-64f;
+    r.up = 0x1p64f;
+    r.s1 = lanes_csum<W>(CSum{a1.s * down, a1.c * down}, mask);
+    if constexpr (TWO) r.s2 = lanes_csum<W>(CSum{a2.s * down, a2.c * down}, mask);
+}
 template <int W, bool TWO> __device__ __forceinline__ void lanes_sums(Sums &r, unsigned mask, bool check)
 {
     const CSum a1 = r.s1, a2 = r.s2;
@@ -546,11 +558,7 @@ template <int W, bool TWO> __device__ __forceinline__ void lanes_sums(Sums &r, u
     if (!check) return;
     bool out = !(r.s1.s - r.s1.s == 0.0f);
     if constexpr (TWO) out |= !(r.s2.s - r.s2.s == 0.0f);
-    if (!__shfl_sync(mask, (int)out, (int)(threadIdx.x & 31 & ~(W - 1)))) return;  // (the first lane's are whole)
-    constexpr float down = 0x1p-64f;
-    r.up = 0x1p64f;
-    r.s1 = lanes_csum<W>(CSum{a1.s * down, a1.c * down}, mask);
-    if constexpr (TWO) r.s2 = lanes_csum<W>(CSum{a2.s * down, a2.c * down}, mask);
+    if (__shfl_sync(mask, (int)out, (int)(threadIdx.x & 31 & ~(W - 1)))) lanes_scaled<W, TWO>(r, a1, a2, mask);
 }
 template <int W> __device__ __forceinline__ double lanes_sum64(double a, unsigned mask)
 {
