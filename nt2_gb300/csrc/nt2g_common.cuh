@@ -31,8 +31,9 @@ inline bool aligned16(const void *p) { return ((uintptr_t)p & 15u) == 0; }
 // launch_dependent() may start while the previous kernel in its stream is
 // still running; pdl_wait() returns once that kernel has completed and its
 // memory is visible (immediately when there is no such dependency).  A kernel
-// reads only inputs no earlier kernel writes before pdl_wait(), and writes
-// nothing before it.  pdl_trigger() lets the next dependent launch begin; at a
+// reads and writes no memory of its arguments before it: what its own predecessor
+// does not write may still be written by one before that, which let both line up.
+// pdl_trigger() lets the next dependent launch begin; at a
 // kernel's start, it lets the next kernel's blocks line up once all of this one's
 // run.  (Folds, their combining kernels and the median's passes: 9 and 8 launches
 // of a table's six statistics and three medians, 286 -> 266 and 142 -> 128 us.)

@@ -84,9 +84,9 @@ __global__ void __launch_bounds__(kFoldThreads, is_var(OP) ? 3 : 4) k_fold_outer
 }
 
 template <int OP, int VEC>
-__global__ void __launch_bounds__(kFoldThreads, VEC == 4 || is_var(OP) || OP == MEANAD ? 4 : 8) k_fold_columns(RawSrc src, int64_t lo, int64_t inner, int64_t hi,
-                                                             float *__restrict__ out, int64_t *__restrict__ index,
-                                                             const float *__restrict__ cen, double *__restrict__ out64)
+__global__ void __launch_bounds__(kFoldThreads, VEC == 4 || is_var(OP) || OP == MEANAD ? 4 : 8)
+k_fold_columns(RawSrc src, int64_t lo, int64_t inner, int64_t hi, float *__restrict__ out, int64_t *__restrict__ index,
+               const float *__restrict__ cen, double *__restrict__ out64)
 {
     pdl_trigger();
     pdl_wait_for(src.x, out, index, cen, out64);
@@ -248,7 +248,7 @@ static FoldPlan plan_fold(int64_t lo, int64_t inner, int64_t hi, bool aligned, i
         return p;
     }
     const int64_t columns = (lo * hi / p.vec + 31) / 32;  // blocks side by side
-    // (a variance's partials cost some twenty FP64 instructions each to combine)
+    // (a variance's partials cost some ten FP64 instructions each to combine)
     int64_t q = ((is_var(op) ? kBlocks / 2 : kBlocks) + columns - 1) / columns;
     const int64_t qmax = inner / 64 > 0 ? inner / 64 : 1;  // eight rows a warp at least
     if (q > qmax) q = qmax;
@@ -430,8 +430,11 @@ static nt2g_status launch_fold_op(const FoldInput &in, int64_t lo, int64_t inner
     } else if (p.kind == 3) {
         const dim3 g(cap((n_out / p.vec + kFoldThreads - 1) / kFoldThreads));
         if (!in.expr) {
-            if (!is_var(OP) && p.vec == 4) ce = launch_dependent(k_fold_columns<OP, is_var(OP) ? 1 : 4>, g, kFoldThreads, st, src, lo, inner, hi, out, index, cen, out64);
-            else ce = launch_dependent(k_fold_columns<OP, 1>, g, kFoldThreads, st, src, lo, inner, hi, out, index, cen, out64);
+            if (!is_var(OP) && p.vec == 4)
+                ce = launch_dependent(k_fold_columns<OP, is_var(OP) ? 1 : 4>, g, kFoldThreads, st, src, lo, inner, hi, out,
+                                      index, cen, out64);
+            else
+                ce = launch_dependent(k_fold_columns<OP, 1>, g, kFoldThreads, st, src, lo, inner, hi, out, index, cen, out64);
         } else {
             void *pr[] = {(void *)jargs, &lo, &inner, &hi, &out, &index, &cen, &out64};
             ce = launch_by_handle(jk->columns[p.vec == 4], g, pr, st);

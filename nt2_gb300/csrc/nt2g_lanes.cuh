@@ -1,6 +1,7 @@
 // nt2g_lanes.cuh -- the fast policy's functions over the lanes a thread holds
-// (4 or 8 consecutive elements in the run-time compiled kernels), two lanes per
-// packed instruction, the special values handled once for all lanes: a thread
+// (in the run-time compiled kernels 4 consecutive elements of a transform, 4 or
+// 8 of a batch item, 1 or 4 of a fold, 2 of reverse mode), two lanes per packed
+// instruction, the special values handled once for all lanes: a thread
 // first asks whether any of its lanes is outside the common range of the
 // function, and if one is, all its lanes take the scalar function.  Within the
 // common range each lane performs exactly the operations of the scalar
@@ -54,7 +55,8 @@ __device__ __forceinline__ f2 erfc_tail_poly2(f2 w)
 
 // 1/b correctly rounded for normal b whose reciprocal is normal (what
 // Fast::div(1, b) gives): one Newton step on the SFU's reciprocal rounds
-// correctly for every significand (checked over all 2^23).
+// correctly for every significand (tested over all 2^23, through gammaln, log1p
+// and pow).
 __device__ __forceinline__ f2 recip_rn2(f2 b)
 {
     const f2 nb = negx2(b), y = lanes(b, [](float v) { return Fast::rcp(v); });

@@ -166,7 +166,7 @@ def check(status):
 
 
 # A call through this binding is a microsecond or two of checks and launch in
-# the library; what follows keeps the Python side near that (3.7 us a call in
+# the library; what follows keeps the Python side near that (4.6 us a call in
 # all on the GB300's Grace, 9.4 with a torch Stream object and a ctypes object
 # per pointer).  Addresses cross as Python integers.
 def _ptr(t):
